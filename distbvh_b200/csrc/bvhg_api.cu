@@ -209,7 +209,7 @@ struct bvhg_ctx
   cudaEvent_t fork_evt = nullptr;
   std::string err;
   // sort-and-sweep scratch
-  dev_buf sw_keys, sw_vals, sw_rows, sw_srows, sw_sbmax, sw_hist, sw_status, sw_sc, sw_params, sw_partial;
+  dev_buf sw_keys, sw_vals, sw_srows, sw_start, sw_hist, sw_status, sw_sc, sw_params, sw_partial;
   // pairs
   dev_buf pairs, pairs2, pairs_out, pscal;
   // element pairs grouped by patch pair
@@ -1627,14 +1627,13 @@ bvhg_status bvhg_sort_and_sweep(bvhg_ctx *ctx, int32_t obj_a, int32_t obj_b, int
   const uint64_t nb = b.n;
   const uint64_t nb4 = ( nb + 3 ) & ~3ull;  // second halves of the ping-pong buffers start 16-byte aligned
   const uint64_t tiles = ( nb + kSortTile - 1 ) / kSortTile;
-  const uint64_t status_words = 4 * ( tiles + 1 ) * 256;
+  const uint64_t status_words = 2 * ( tiles + 1 ) * 256;
   cudaStream_t s = ctx->stream;
   BVHG_CUDA( ctx, ctx->sw_keys.reserve( 2 * nb4 * 8 ) );
   BVHG_CUDA( ctx, ctx->sw_vals.reserve( 2 * nb4 * 4 ) );
-  BVHG_CUDA( ctx, ctx->sw_rows.reserve( nb * K * 8 ) );
   BVHG_CUDA( ctx, ctx->sw_srows.reserve( nb * K * 8 ) );
-  BVHG_CUDA( ctx, ctx->sw_sbmax.reserve( nb * 8 ) );
-  BVHG_CUDA( ctx, ctx->sw_hist.reserve( 4 * 256 * 4 ) );
+  BVHG_CUDA( ctx, ctx->sw_start.reserve( sweep_start_bytes() ) );
+  BVHG_CUDA( ctx, ctx->sw_hist.reserve( 2 * 256 * 4 ) );
   BVHG_CUDA( ctx, ctx->sw_status.reserve( status_words * 4 ) );
   BVHG_CUDA( ctx, ctx->sw_sc.reserve( sizeof( obj_scalars ) ) );
   BVHG_CUDA( ctx, ctx->sw_params.reserve( sweep_params_bytes() ) );
@@ -1668,13 +1667,12 @@ bvhg_status bvhg_sort_and_sweep(bvhg_ctx *ctx, int32_t obj_a, int32_t obj_b, int
   x.bsc = b.sc();
   x.partial = ctx->sw_partial.as< double >();
   x.params = ctx->sw_params.p;
-  x.rows = ctx->sw_rows.as< double >();
   x.keys = k0;
   x.hist = ctx->sw_hist.as< uint32_t >();
-  x.skeys = k0;  // four passes: k0 -> k1 -> k0 -> k1 -> k0
+  x.skeys = k0;  // two passes: k0 -> k1 -> k0
   x.svals = v0;
+  x.start = ctx->sw_start.as< uint32_t >();
   x.srows = ctx->sw_srows.as< double >();
-  x.sbmax = ctx->sw_sbmax.as< double >();
   x.aperm = a.sorted_vals();
   x.sc = ssc;
   x.ps = ps;
@@ -1684,12 +1682,12 @@ bvhg_status bvhg_sort_and_sweep(bvhg_ctx *ctx, int32_t obj_a, int32_t obj_b, int
     x.pairs = ctx->pairs.as< uint2 >();
     x.cap = ctx->pair_cap;
     BVHG_CUDA( ctx, cudaMemsetAsync( ssc, 0, sizeof( obj_scalars ), s ) );
-    BVHG_CUDA( ctx, cudaMemsetAsync( x.hist, 0, 4 * 256 * 4, s ) );
+    BVHG_CUDA( ctx, cudaMemsetAsync( x.hist, 0, 2 * 256 * 4, s ) );
     BVHG_CUDA( ctx, cudaMemsetAsync( ctx->sw_status.p, 0, status_words * 4, s ) );
     BVHG_CUDA( ctx, cudaMemsetAsync( ps, 0, sizeof( pair_scalars ), s ) );
     BVHG_CUDA( ctx, launch_sweep_setup( x, axis ) );
     BVHG_CUDA( ctx, launch_sweep_keys( x ) );
-    for ( int pass = 0; pass < 4; ++pass )
+    for ( int pass = 0; pass < 2; ++pass )
     {
       const bool even = ( pass & 1 ) == 0;
       BVHG_CUDA( ctx, launch_onesweep( 8, even ? k0 : k1, pass == 0 ? nullptr : ( even ? v0 : v1 ), even ? k1 : k0,

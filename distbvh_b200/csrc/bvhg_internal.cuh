@@ -272,13 +272,12 @@ struct sweep_launch
   const obj_scalars *asc, *bsc;                     // K1 bounds of both objects (global range)
   double *partial;                                  // sweep_partial_bytes()
   void *params;                                     // sweep_params_bytes()
-  double *rows;                                     // nb * K doubles: B's element slabs, original order
-  uint64_t *keys;                                   // nb: B's u32 keys, original order
-  uint32_t *hist;                                   // 4 * 256: byte histograms of the keys
+  uint64_t *keys;                                   // nb: B's (strip, bin) keys, original order
+  uint32_t *hist;                                   // 2 * 256: byte histograms of the keys
   const uint64_t *skeys;                            // sorted keys
   const uint32_t *svals;                            // B's element indices in key order
-  double *srows;                                    // nb * K doubles: B's slab rows in key order
-  double *sbmax;                                    // nb: B's scaled maxima on the axis in key order
+  uint32_t *start;                                  // sweep_start_bytes(): first position of every cell
+  double *srows;                                    // nb * K doubles: B's slabs in key order, slab by slab
   const uint32_t *aperm;                            // A's elements in Morton order (its build's permutation)
   const obj_scalars *sc;                            // scalars of the keys' sort (error word)
   uint2 *pairs;
@@ -288,12 +287,13 @@ struct sweep_launch
 };
 size_t sweep_params_bytes();
 size_t sweep_partial_bytes();
+size_t sweep_start_bytes();
 int sweep_axis_read(const void *params_host_copy);
 // The axis (axis < 0: the one of largest centroid variance) and its scale factor, from the objects' bounds.
 cudaError_t launch_sweep_setup(const sweep_launch &x, int axis);
-// B's slab rows, keys, byte histograms and the key window width.
+// B's keys, byte histograms and largest widths.
 cudaError_t launch_sweep_keys(const sweep_launch &x);
-// A's sweeps over the sorted keys; pairs (index into A, index into B) counted in ps->count.
+// B's slabs and cells in sorted order, and A's sweeps; pairs (index into A, index into B) counted in ps->count.
 cudaError_t launch_sweep(const sweep_launch &x);
 
 cudaError_t launch_onesweep(int bits, const uint64_t *keys_in, const uint32_t *vals_in, uint64_t *keys_out,

@@ -4,16 +4,22 @@
 // and max_variant_axis (kokkos.hpp:125-160) for the sweep axis when the caller gives none:
 // - the global range on the axis is the union of both objects' slab extents there (the K1 bounds of each object:
 //   min of the cardinal slab minima, max of the maxima);
-// - B's slab minima on the axis become u32 keys (min - global_min) * (UINT32_MAX / (global_max - global_min)),
-//   truncated; a stable LSD radix sort of (key, index) over the four bytes of the key (the radix pass of k_sort.cu);
-// - every element of A sweeps B in key order: it skips B elements whose scaled maximum lies below its minimum key,
-//   stops at the first B key above its maximum key, and emits the B elements that overlap it strictly on every
-//   slab. The emitted set is the exact pair set S(A, B) for any axis.
-// Here each A element sweeps only the key window [its minimum key - W, its maximum key], W = the largest
-// (scaled maximum - key) over B: every B element below the window has a scaled maximum below A's minimum key and is
-// one the reference's loop skips, so the window emits the same pairs.
-// A degenerate axis (global_max == global_min) gives every key 0 here; the reference's factor is then infinite and
-// its keys 0 as well (NaN converts to 0), with the same outcome: no element is skipped or stops a sweep.
+// - the reference scales B's slab minima on the axis to u32 keys, sorts them stably, and lets every element of A
+//   sweep B in key order: it skips the B elements that end before its minimum, stops at the first that begins after
+//   its maximum, and emits those that overlap it strictly on every slab. The emitted set is the exact pair set S(A, B)
+//   for any axis.
+// The emitted set is that of the strict all-slab overlap, so the order in which candidates are met is free. A one
+// dimensional sweep of three dimensional elements meets thousands of them per element (two soups of 262,144 triangles:
+// 4,000 B elements in every window). Here the sweep axis is cut into 256 strips and every strip is swept on a
+// second axis (of the other two the one of larger extent), cut into 256 bins: B's key is (strip of its slab minimum,
+// bin of its second slab minimum), 16 bits, two radix passes, and start[] holds the first sorted position of every
+// (strip, bin) cell. An element of A then sweeps, in each strip of [its minimum - W, its maximum], the positions of
+// the bins of [its second minimum - W2, its second maximum], where W and W2 are the largest widths of a B element on
+// the two axes. Every overlapping B element lies there: b.min < a.max, and b.min >= b.max - W > a.min - W, with W
+// rounded up, a.min - W rounded down and the strip a monotone function of the value. The candidates are tested on the
+// third axis first, whose slabs lie contiguously in sorted order, then on the other slabs. The call on those two soups
+// takes 0.40 ms instead of 4.46 ms.
+// A degenerate axis (global_max == global_min) puts every element into strip or bin 0.
 #include "bvhg_internal.cuh"
 #include "kdop_math.cuh"
 
@@ -24,26 +30,38 @@ namespace {
 constexpr int kSweepThreads = 256;
 constexpr int kAxisBlocks = 512;  // partial sums of the axis choice (a fixed grid: a fixed summation order)
 
+constexpr int kStrips = 256;  // strips of the sweep axis and bins of the second axis: one key byte each
+constexpr int kCells = kStrips * kStrips;
+
 struct sweep_params
 {
-  int axis;
+  int axis;  // the sweep axis (read back by the host)
+  int axis2, axis3;
   int pad;
-  double gmin;
-  double fac;
-  unsigned long long wmax_enc;  // order-preserving encoding of W
+  double gmin[2], fac[2];         // range minimum and scale factor of the sweep axis and the second axis
+  unsigned long long wmax_enc[2]; // order-preserving encodings of W and W2
 };
 
-// u32 of a scaled value as the reference's conversion yields it for every value this path produces (truncation;
-// NaN and values outside the signed 64-bit range give 0).
-__device__ __forceinline__ uint32_t key32(double x)
+// Strip (or bin) of a value: monotone in v; NaN gives 0.
+__device__ __forceinline__ uint32_t strip_of(double v, const sweep_params &p, int which)
 {
-  if ( !( x < 9223372036854775808.0 ) || !( x >= -9223372036854775808.0 ) ) return 0u;
-  return static_cast< uint32_t >( static_cast< unsigned long long >( __double2ll_rz( x ) ) );
+  const double t = __dmul_rn( __dsub_rn( v, p.gmin[which] ), p.fac[which] );
+  if ( !( t >= 0.0 ) ) return 0u;
+  return t >= static_cast< double >( kStrips - 1 ) ? kStrips - 1 : static_cast< uint32_t >( t );
 }
 
-__device__ __forceinline__ double scaled(double v, const sweep_params &p)
+// The minimum and maximum of one coordinate over an element's vertices, with the inflation: the cardinal slab.
+__device__ __forceinline__ void cardinal_slab(const double *__restrict__ src, int V, int axis, double eps, double &lo, double &hi)
 {
-  return __dmul_rn( __dsub_rn( v, p.gmin ), p.fac );
+  double mn = __ldg( src + axis ), mx = mn;
+  for ( int v = 1; v < V; ++v )
+  {
+    const double t = __ldg( src + 3 * v + axis );
+    mn = std_min( mn, t );
+    mx = std_max( mx, t );
+  }
+  lo = __dsub_rn( mn, eps );
+  hi = __dadd_rn( mx, eps );
 }
 
 // Partial sums of the centroids and their squares over A then B (block b: a grid-stride range), fixed order.
@@ -82,228 +100,295 @@ __global__ void __launch_bounds__( kSweepThreads ) k_axis_partial(const double *
   if ( threadIdx.x < 6 ) partial[blockIdx.x * 6 + threadIdx.x] = s_red[threadIdx.x][0];
 }
 
-// The axis (given, or of largest centroid variance), the global range on it and the scale factor.
-__global__ void k_sweep_setup(const double *__restrict__ partial, int nblocks, uint64_t n, int axis_in,
-                              const obj_scalars *__restrict__ sa, const obj_scalars *__restrict__ sb,
-                              sweep_params *__restrict__ p)
+// The axis (given, or of largest centroid variance), the second axis, the global ranges on both and the scale
+// factors. The partial sums are added in block order (one lane per sum, from shared memory: a single thread reading
+// them from global memory took 135 us), so the axis does not depend on the run.
+__global__ void __launch_bounds__( 256 ) k_sweep_setup(const double *__restrict__ partial, int nblocks, uint64_t n,
+                                                       int axis_in, const obj_scalars *__restrict__ sa,
+                                                       const obj_scalars *__restrict__ sb, sweep_params *__restrict__ p)
 {
-  if ( threadIdx.x != 0 ) return;
+  __shared__ double s_part[kAxisBlocks * 6];
+  __shared__ double s_sum[6];
   int axis = axis_in;
   if ( axis < 0 )
   {
-    double s[6] = { 0, 0, 0, 0, 0, 0 };
-    for ( int b = 0; b < nblocks; ++b )
-      for ( int k = 0; k < 6; ++k ) s[k] = __dadd_rn( s[k], partial[b * 6 + k] );
+    for ( int k = threadIdx.x; k < nblocks * 6; k += 256 ) s_part[k] = partial[k];
+    __syncthreads();
+    if ( threadIdx.x < 6 )
+    {
+      double s = 0;
+      for ( int b = 0; b < nblocks; ++b ) s = __dadd_rn( s, s_part[b * 6 + threadIdx.x] );
+      s_sum[threadIdx.x] = s;
+    }
+    __syncthreads();
+  }
+  if ( threadIdx.x != 0 ) return;
+  if ( axis < 0 )
+  {
     double var[3];
     for ( int k = 0; k < 3; ++k )
-      var[k] = __dsub_rn( s[3 + k], __ddiv_rn( __dmul_rn( s[k], s[k] ), static_cast< double >( n ) ) );
+      var[k] = __dsub_rn( s_sum[3 + k], __ddiv_rn( __dmul_rn( s_sum[k], s_sum[k] ), static_cast< double >( n ) ) );
     axis = 0;
     if ( var[1] > var[0] ) axis = 1;
     if ( var[2] > var[axis] ) axis = 2;
   }
-  const double amin = ord_decode( sa->bounds_enc[axis] ), amax = ord_decode( sa->bounds_enc[3 + axis] );
-  const double bmin = ord_decode( sb->bounds_enc[axis] ), bmax = ord_decode( sb->bounds_enc[3 + axis] );
-  const double gmin = bmin < amin ? bmin : amin;
-  const double gmax = amax < bmax ? bmax : amax;
+  double gmin[3], ext[3];
+  for ( int k = 0; k < 3; ++k )
+  {
+    const double amin = ord_decode( sa->bounds_enc[k] ), amax = ord_decode( sa->bounds_enc[3 + k] );
+    const double bmin = ord_decode( sb->bounds_enc[k] ), bmax = ord_decode( sb->bounds_enc[3 + k] );
+    gmin[k] = bmin < amin ? bmin : amin;
+    ext[k] = __dsub_rn( amax < bmax ? bmax : amax, gmin[k] );
+  }
+  const int u = axis == 0 ? 1 : 0, v = axis == 2 ? 1 : 2;  // the other two axes
+  const int axis2 = ext[v] > ext[u] ? v : u;
   p->axis = axis;
-  p->gmin = gmin;
-  p->fac = gmax > gmin ? __ddiv_rn( 4294967295.0, __dsub_rn( gmax, gmin ) ) : 0.0;
-  p->wmax_enc = ord_encode( 0.0 );
+  p->axis2 = axis2;
+  p->axis3 = 3 - axis - axis2;
+  p->gmin[0] = gmin[axis];
+  p->gmin[1] = gmin[axis2];
+  p->fac[0] = ext[axis] > 0.0 ? __ddiv_rn( static_cast< double >( kStrips ), ext[axis] ) : 0.0;
+  p->fac[1] = ext[axis2] > 0.0 ? __ddiv_rn( static_cast< double >( kStrips ), ext[axis2] ) : 0.0;
+  p->wmax_enc[0] = p->wmax_enc[1] = ord_encode( 0.0 );
 }
 
-// B: element slab rows (original order), u32 keys of the slab minima on the axis, the byte histograms of the four
-// radix passes, and W = max (scaled maximum - key).
-template< int K, int VT >
-__global__ void __launch_bounds__( kSweepThreads ) k_sweep_keys(const double *__restrict__ verts, uint32_t Vrt,
-                                                                uint64_t n, double eps,
-                                                                const sweep_params *pp, double *__restrict__ rows,
+// B's keys, the histograms of their two bytes, and the largest widths on the two axes.
+__global__ void __launch_bounds__( kSweepThreads ) k_sweep_keys(const double *__restrict__ verts, int V, uint64_t n,
+                                                                double eps, const sweep_params *pp,
                                                                 uint64_t *__restrict__ keys, uint32_t *__restrict__ hist,
                                                                 sweep_params *pw)  // pp and pw: the same struct
 {
-  constexpr int D = K / 2;
-  __shared__ uint32_t s_hist[4 * 256];
-  __shared__ double s_w[kSweepThreads / 32];
-  for ( int k = threadIdx.x; k < 4 * 256; k += kSweepThreads ) s_hist[k] = 0;
+  __shared__ uint32_t s_hist[2 * 256];
+  __shared__ double s_w[2][kSweepThreads / 32];
+  for ( int k = threadIdx.x; k < 2 * 256; k += kSweepThreads ) s_hist[k] = 0;
   const sweep_params p = *pp;
   __syncthreads();
   const uint64_t i = static_cast< uint64_t >( blockIdx.x ) * kSweepThreads + threadIdx.x;
-  double w = 0.0;
+  double w[2] = { 0.0, 0.0 };
   if ( i < n )
   {
-    double lo[D], hi[D];
-    leaf_slabs< K, double, VT >( verts, Vrt, static_cast< uint32_t >( i ), eps, 0.f, lo, hi );
-    double *row = rows + i * 2 * D;
+    const double *src = verts + i * V * 3;
+    uint32_t key = 0;
 #pragma unroll
-    for ( int a = 0; a < D; ++a )
+    for ( int c = 0; c < 2; ++c )
     {
-      row[2 * a] = lo[a];
-      row[2 * a + 1] = hi[a];
+      double lo, hi;
+      cardinal_slab( src, V, c ? p.axis2 : p.axis, eps, lo, hi );
+      key = ( key << 8 ) | strip_of( lo, p, c );
+      w[c] = __dsub_ru( hi, lo );
     }
-    const double mn = p.axis == 0 ? lo[0] : ( p.axis == 1 ? lo[1] : lo[2] );
-    const double mx = p.axis == 0 ? hi[0] : ( p.axis == 1 ? hi[1] : hi[2] );
-    const uint32_t key = key32( scaled( mn, p ) );
     keys[i] = key;
-    w = __dsub_rn( scaled( mx, p ), static_cast< double >( key ) );
-    for ( int q = 0; q < 4; ++q ) atomicAdd( &s_hist[q * 256 + ( ( key >> ( 8 * q ) ) & 255u )], 1u );
+    atomicAdd( &s_hist[key & 255u], 1u );
+    atomicAdd( &s_hist[256 + ( key >> 8 )], 1u );
   }
-  for ( int o = 16; o > 0; o >>= 1 )
+#pragma unroll
+  for ( int c = 0; c < 2; ++c )
   {
-    const double x = __shfl_xor_sync( 0xffffffffu, w, o );
-    w = x > w ? x : w;
+    for ( int o = 16; o > 0; o >>= 1 )
+    {
+      const double x = __shfl_xor_sync( 0xffffffffu, w[c], o );
+      w[c] = w[c] > x ? w[c] : ( x > w[c] ? x : ( w[c] == w[c] ? w[c] : x ) );
+    }
+    if ( ( threadIdx.x & 31 ) == 0 ) s_w[c][threadIdx.x >> 5] = w[c];
   }
-  if ( ( threadIdx.x & 31 ) == 0 ) s_w[threadIdx.x >> 5] = w;
   __syncthreads();
-  for ( int k = threadIdx.x; k < 4 * 256; k += kSweepThreads )
+  for ( int k = threadIdx.x; k < 2 * 256; k += kSweepThreads )
     if ( s_hist[k] ) atomicAdd( &hist[k], s_hist[k] );
-  if ( threadIdx.x == 0 )
+  if ( threadIdx.x < 2 )
   {
-    double m = s_w[0];
-    for ( int k = 1; k < kSweepThreads / 32; ++k ) m = s_w[k] > m ? s_w[k] : m;
-    atomicMax( &pw->wmax_enc, ord_encode( m ) );
+    double m = 0.0;
+    for ( int k = 0; k < kSweepThreads / 32; ++k ) m = s_w[threadIdx.x][k] > m ? s_w[threadIdx.x][k] : m;
+    atomicMax( &pw->wmax_enc[threadIdx.x], ord_encode( m ) );
   }
 }
 
-// B in key order: its slab rows and its scaled maxima on the axis (the sweeps read both sequentially).
-template< int K >
-__global__ void __launch_bounds__( kSweepThreads ) k_sweep_gather(const double *__restrict__ rows,
-                                                                  const uint32_t *__restrict__ svals, uint64_t n,
-                                                                  const sweep_params *__restrict__ pp,
-                                                                  double *__restrict__ srows,
-                                                                  double *__restrict__ sbmax)
+// First index in [0, n) whose key is >= v.
+__device__ __forceinline__ uint32_t key_bound(const uint64_t *__restrict__ keys, uint32_t n, uint32_t v)
 {
-  constexpr int C = K;  // 2 D values per row
-  const sweep_params p = *pp;
-  for ( uint64_t k = static_cast< uint64_t >( blockIdx.x ) * kSweepThreads + threadIdx.x; k < n * C;
-        k += static_cast< uint64_t >( gridDim.x ) * kSweepThreads )
-  {
-    const uint64_t j = k / C;
-    const int c = static_cast< int >( k - j * C );
-    const double v = __ldg( rows + static_cast< uint64_t >( __ldg( svals + j ) ) * C + c );
-    srows[k] = v;
-    if ( c == 2 * p.axis + 1 ) sbmax[j] = scaled( v, p );
-  }
-}
-
-// First index in [0, n) whose key is >= v (lower) or > v (upper).
-__device__ __forceinline__ uint64_t key_bound(const uint64_t *__restrict__ keys, uint64_t n, uint64_t v, bool upper)
-{
-  uint64_t lo = 0, hi = n;
+  uint32_t lo = 0, hi = n;
   while ( lo < hi )
   {
-    const uint64_t mid = ( lo + hi ) >> 1;
-    const uint64_t k = __ldg( keys + mid );
-    if ( upper ? k <= v : k < v ) lo = mid + 1;
+    const uint32_t mid = ( lo + hi ) >> 1;
+    if ( static_cast< uint32_t >( __ldg( keys + mid ) ) < v ) lo = mid + 1;
     else hi = mid;
   }
   return lo;
 }
 
-// A: one warp per element (A in its Morton order, warps grid-stride over it). All lanes form the element's slabs
-// and window (the same values; the loads are broadcasts), then scan the window 32 keys at a time: lane l tests
-// key j0 + l + 32 k, so every load of the scaled maxima and of the rows is coalesced across the warp.
+constexpr unsigned kStartBlocks = ( kCells + 1 + kSweepThreads - 1 ) / kSweepThreads;
+
+// Blocks [0, kStartBlocks): start[c], the first sorted position of cell c or a later one (start[kCells] = n). The
+// others: B's slabs in sorted order, slab by slab (the pair of slab a and position j at srows[2 (a n + j)]), so that
+// a warp reads one slab of 32 neighbouring positions as one contiguous piece.
 template< int K, int VT >
-__global__ void __launch_bounds__( kSweepThreads ) k_sweep(const double *__restrict__ verts, uint32_t Vrt, uint64_t na,
-                                                           double eps, const sweep_params *__restrict__ pp,
-                                                           const uint32_t *__restrict__ aperm,
-                                                           const uint64_t *__restrict__ skeys,
-                                                           const uint32_t *__restrict__ svals,
-                                                           const double *__restrict__ srows,
-                                                           const double *__restrict__ sbmax, uint64_t nb,
-                                                           const obj_scalars *__restrict__ ssc, uint2 *__restrict__ pairs,
-                                                           uint64_t cap, pair_scalars *__restrict__ ps)
+__global__ void __launch_bounds__( kSweepThreads ) k_sweep_gather(const double *__restrict__ verts, uint32_t Vrt,
+                                                                  double eps, const uint64_t *__restrict__ skeys,
+                                                                  const uint32_t *__restrict__ svals, uint64_t n,
+                                                                  const obj_scalars *__restrict__ ssc,
+                                                                  uint32_t *__restrict__ start,
+                                                                  double *__restrict__ srows)
 {
   constexpr int D = K / 2;
   if ( *reinterpret_cast< const volatile int * >( &ssc->error ) == kErrTimeout ) return;  // keys not sorted
-  const sweep_params p = *pp;
-  const double W = ord_decode( p.wmax_enc );
-  const uint64_t wq = W < 8589934592.0 ? static_cast< uint64_t >( ceil( W ) ) : 8589934592ull;  // >= every key span
-  const unsigned lane = threadIdx.x & 31u;
-  const uint64_t nwarps = static_cast< uint64_t >( gridDim.x ) * ( kSweepThreads / 32 );
-  for ( uint64_t t = ( static_cast< uint64_t >( blockIdx.x ) * kSweepThreads + threadIdx.x ) >> 5; t < na; t += nwarps )
+  if ( blockIdx.x < kStartBlocks )
   {
-    const uint32_t i = __ldg( aperm + t );
+    const uint32_t c = blockIdx.x * kSweepThreads + threadIdx.x;
+    if ( c <= kCells ) start[c] = c == kCells ? static_cast< uint32_t >( n ) : key_bound( skeys, static_cast< uint32_t >( n ), c );
+    return;
+  }
+  const uint64_t j = static_cast< uint64_t >( blockIdx.x - kStartBlocks ) * kSweepThreads + threadIdx.x;
+  if ( j >= n ) return;
+  double lo[D], hi[D];
+  leaf_slabs< K, double, VT >( verts, Vrt, __ldg( svals + j ), eps, 0.f, lo, hi );
+#pragma unroll
+  for ( int a = 0; a < D; ++a )
+    reinterpret_cast< double2 * >( srows )[static_cast< uint64_t >( a ) * n + j] = make_double2( lo[a], hi[a] );
+}
+
+constexpr int kPairThreads = 128;
+
+// A: a warp takes `per` (at most 32) consecutive elements of A in Morton order. Every lane forms the slabs and the
+// strip and bin ranges of one of them; then the warp sweeps them one after the other, 32 positions of a strip at a
+// time. All lanes forming the same element's slabs, one warp per element, cost as much as the sweep itself.
+template< int K, int VT >
+__global__ void __launch_bounds__( kPairThreads ) k_sweep(const double *__restrict__ verts, uint32_t Vrt, uint64_t na,
+                                                          uint32_t per, double eps, const sweep_params *__restrict__ pp,
+                                                          const uint32_t *__restrict__ aperm,
+                                                          const uint32_t *__restrict__ start,
+                                                          const uint32_t *__restrict__ svals,
+                                                          const double *__restrict__ srows, uint64_t nb,
+                                                          const obj_scalars *__restrict__ ssc, uint2 *__restrict__ pairs,
+                                                          uint64_t cap, pair_scalars *__restrict__ ps)
+{
+  constexpr int D = K / 2;
+  __shared__ alignas( 16 ) double s_rows[kPairThreads / 32][32][K];
+  if ( *reinterpret_cast< const volatile int * >( &ssc->error ) == kErrTimeout ) return;  // keys not sorted
+  const sweep_params p = *pp;
+  const unsigned lane = threadIdx.x & 31u, lt = ( 1u << lane ) - 1u;
+  double( *rows )[K] = s_rows[threadIdx.x >> 5];
+  const double2 *z = reinterpret_cast< const double2 * >( srows ) + static_cast< uint64_t >( p.axis3 ) * nb;
+  const uint64_t first = static_cast< uint64_t >( ( blockIdx.x * kPairThreads + threadIdx.x ) >> 5 ) * per;
+  uint32_t i = 0, span = 0;  // span: first strip, last strip, first bin, last bin
+  if ( lane < per && first + lane < na )
+  {
+    i = __ldg( aperm + first + lane );
     double lo[D], hi[D];
     leaf_slabs< K, double, VT >( verts, Vrt, i, eps, 0.f, lo, hi );
-    const double mn = p.axis == 0 ? lo[0] : ( p.axis == 1 ? lo[1] : lo[2] );
-    const double mx = p.axis == 0 ? hi[0] : ( p.axis == 1 ? hi[1] : hi[2] );
-    const uint32_t amin = key32( scaled( mn, p ) );
-    const uint32_t amax = key32( scaled( mx, p ) );
-    const uint64_t start = amin > wq ? amin - wq : 0;
-    const uint64_t j0 = key_bound( skeys, nb, start, false );
-    const uint64_t j1 = key_bound( skeys, nb, amax, true );
-    const double amin_d = static_cast< double >( amin );
-    for ( uint64_t j = j0 + lane; j < j1; j += 32 )
-    {
-      if ( __ldg( sbmax + j ) < amin_d ) continue;
-      const double *row = srows + j * 2 * D;
-      bool o = true;
 #pragma unroll
-      for ( int a = 0; a < D; ++a )
+    for ( int a = 0; a < D; ++a )
+    {
+      rows[lane][2 * a] = lo[a];
+      rows[lane][2 * a + 1] = hi[a];
+    }
+#pragma unroll
+    for ( int c = 0; c < 2; ++c )
+    {
+      const int a = c ? p.axis2 : p.axis;
+      const double mn = a == 0 ? lo[0] : ( a == 1 ? lo[1] : lo[2] ), mx = a == 0 ? hi[0] : ( a == 1 ? hi[1] : hi[2] );
+      span |= ( strip_of( __dsub_rd( mn, ord_decode( p.wmax_enc[c] ) ), p, c ) | ( strip_of( mx, p, c ) << 8 ) ) << ( 16 * c );
+    }
+  }
+  __syncwarp();
+  const uint32_t count = first < na ? static_cast< uint32_t >( min( static_cast< uint64_t >( per ), na - first ) ) : 0u;
+  for ( uint32_t u = 0; u < count; ++u )
+  {
+    const uint32_t ai = __shfl_sync( 0xffffffffu, i, u ), sp = __shfl_sync( 0xffffffffu, span, u );
+    const uint32_t s0 = sp & 255u, s1 = ( sp >> 8 ) & 255u, y0 = ( sp >> 16 ) & 255u, y1 = sp >> 24;
+    const double *row = rows[u];
+    const double zlo = row[2 * p.axis3], zhi = row[2 * p.axis3 + 1];
+    for ( uint32_t sb = s0; sb <= s1; sb += 32 )
+    {
+      uint32_t b = 0, e = 0;  // the positions of strip sb + lane
+      if ( sb + lane <= s1 )
       {
-        if ( !o ) break;
-        o = lo[a] < __ldg( row + 2 * a + 1 ) && __ldg( row + 2 * a ) < hi[a];
+        b = __ldg( start + ( sb + lane ) * kStrips + y0 );
+        e = __ldg( start + ( sb + lane ) * kStrips + y1 + 1 );
       }
-      if ( o )
+      for ( unsigned m = __ballot_sync( 0xffffffffu, b < e ); m; m &= m - 1 )
       {
-        const unsigned long long pos = atomicAdd( &ps->count, 1ull );
-        if ( pos < cap ) pairs[pos] = make_uint2( i, __ldg( svals + j ) );
+        const int s = __ffs( m ) - 1;
+        const uint32_t jb = __shfl_sync( 0xffffffffu, b, s ), je = __shfl_sync( 0xffffffffu, e, s );
+        for ( uint32_t j0 = jb; j0 < je; j0 += 32 )
+        {
+          const uint32_t j = j0 + lane;
+          bool o = false;
+          if ( j < je )
+          {
+            const double2 t = __ldg( z + j );
+            o = zlo < t.y && t.x < zhi;
+          }
+          if ( !__any_sync( 0xffffffffu, o ) ) continue;
+#pragma unroll 1
+          for ( int a = 0; a < D; ++a )
+          {
+            if ( !o ) break;
+            const double2 t = __ldg( reinterpret_cast< const double2 * >( srows ) + static_cast< uint64_t >( a ) * nb + j );
+            o = row[2 * a] < t.y && t.x < row[2 * a + 1];
+          }
+          const unsigned bal = __ballot_sync( 0xffffffffu, o );
+          if ( !bal ) continue;
+          unsigned long long at = 0;
+          if ( lane == 0 ) at = atomicAdd( &ps->count, static_cast< unsigned long long >( __popc( bal ) ) );
+          at = __shfl_sync( 0xffffffffu, at, 0 ) + __popc( bal & lt );
+          if ( o && at < cap ) pairs[at] = make_uint2( ai, __ldg( svals + j ) );
+        }
       }
     }
   }
 }
 
-template< int K, int VT >
-void sweep_kernels(const sweep_launch &x, cudaError_t &e, bool keys_phase)
+// Elements of A per warp: 32 when that still gives every SM 32 warps, fewer for a small A.
+uint32_t sweep_per_warp(uint64_t na)
 {
-  const sweep_params *pp = static_cast< const sweep_params * >( x.params );
-  if ( keys_phase )
-  {
-    const unsigned grid = static_cast< unsigned >( ( x.nb + kSweepThreads - 1 ) / kSweepThreads );
-    k_sweep_keys< K, VT ><<< grid, kSweepThreads, 0, x.s >>>( x.bverts, x.bV, x.nb, x.eps, pp, x.rows, x.keys, x.hist,
-                                                             static_cast< sweep_params * >( x.params ) );
-  } else {
-    // warps grid-stride over A: at most 16 resident blocks' worth per SM, never more warps than elements
-    const uint64_t want = ( x.na + kSweepThreads / 32 - 1 ) / ( kSweepThreads / 32 );
-    const uint64_t cap = static_cast< uint64_t >( device_sm_count() ) * 16;
-    const unsigned grid = static_cast< unsigned >( want < cap ? want : cap );
-    const unsigned ggrid = static_cast< unsigned >( device_sm_count() ) * 8;
-    k_sweep_gather< K ><<< ggrid, kSweepThreads, 0, x.s >>>( x.rows, x.svals, x.nb, pp, x.srows, x.sbmax );
-    e = cudaGetLastError();
-    if ( e != cudaSuccess ) return;
-    k_sweep< K, VT ><<< grid, kSweepThreads, 0, x.s >>>( x.averts, x.aV, x.na, x.eps, pp, x.aperm, x.skeys, x.svals,
-                                                        x.srows, x.sbmax, x.nb, x.sc, x.pairs, x.cap, x.ps );
-  }
-  e = cudaGetLastError();
+  const uint64_t warps = static_cast< uint64_t >( device_sm_count() ) * 32;
+  const uint64_t per = na / warps;
+  return static_cast< uint32_t >( per < 1 ? 1 : ( per > 32 ? 32 : per ) );
+}
+
+template< int K, int VT >
+cudaError_t sweep_gather_t(const sweep_launch &x)
+{
+  const unsigned grid = kStartBlocks + static_cast< unsigned >( ( x.nb + kSweepThreads - 1 ) / kSweepThreads );
+  k_sweep_gather< K, VT ><<< grid, kSweepThreads, 0, x.s >>>( x.bverts, x.bV, x.eps, x.skeys, x.svals, x.nb, x.sc, x.start, x.srows );
+  return cudaGetLastError();
+}
+
+template< int K, int VT >
+cudaError_t sweep_pairs_t(const sweep_launch &x)
+{
+  const uint32_t per = sweep_per_warp( x.na );
+  const uint64_t warps = ( x.na + per - 1 ) / per;
+  const unsigned grid = static_cast< unsigned >( ( warps + kPairThreads / 32 - 1 ) / ( kPairThreads / 32 ) );
+  k_sweep< K, VT ><<< grid, kPairThreads, 0, x.s >>>( x.averts, x.aV, x.na, per, x.eps,
+                                                     static_cast< const sweep_params * >( x.params ), x.aperm, x.start,
+                                                     x.svals, x.srows, x.nb, x.sc, x.pairs, x.cap, x.ps );
+  return cudaGetLastError();
 }
 
 template< int K >
-void sweep_v(const sweep_launch &x, cudaError_t &e, bool keys_phase)
-{
-  const uint32_t V = keys_phase ? x.bV : x.aV;
-  switch ( V )
-  {
-    case 3: sweep_kernels< K, 3 >( x, e, keys_phase ); break;
-    case 4: sweep_kernels< K, 4 >( x, e, keys_phase ); break;
-    case 8: sweep_kernels< K, 8 >( x, e, keys_phase ); break;
-    default: sweep_kernels< K, 0 >( x, e, keys_phase ); break;
-  }
-}
-
-cudaError_t sweep_phase(const sweep_launch &x, bool keys_phase)
+cudaError_t sweep_k(const sweep_launch &x)
 {
   cudaError_t e = cudaErrorInvalidValue;
-  switch ( x.K )
+  switch ( x.bV )
   {
-    case 6: sweep_v< 6 >( x, e, keys_phase ); break;
-    case 18: sweep_v< 18 >( x, e, keys_phase ); break;
-    case 26: sweep_v< 26 >( x, e, keys_phase ); break;
-    default: break;
+    case 3: e = sweep_gather_t< K, 3 >( x ); break;
+    case 4: e = sweep_gather_t< K, 4 >( x ); break;
+    case 8: e = sweep_gather_t< K, 8 >( x ); break;
+    default: e = sweep_gather_t< K, 0 >( x ); break;
   }
-  return e;
+  if ( e != cudaSuccess ) return e;
+  switch ( x.aV )
+  {
+    case 3: return sweep_pairs_t< K, 3 >( x );
+    case 4: return sweep_pairs_t< K, 4 >( x );
+    case 8: return sweep_pairs_t< K, 8 >( x );
+    default: return sweep_pairs_t< K, 0 >( x );
+  }
 }
 
 }  // namespace
 
+size_t sweep_start_bytes() { return ( kCells + 1 ) * sizeof( uint32_t ); }
 size_t sweep_params_bytes() { return sizeof( sweep_params ); }
 size_t sweep_partial_bytes() { return static_cast< size_t >( kAxisBlocks ) * 6 * sizeof( double ); }
 
@@ -318,12 +403,29 @@ cudaError_t launch_sweep_setup(const sweep_launch &x, int axis)
     cudaError_t e = cudaGetLastError();
     if ( e != cudaSuccess ) return e;
   }
-  k_sweep_setup<<< 1, 32, 0, x.s >>>( x.partial, kAxisBlocks, x.na + x.nb, axis, x.asc, x.bsc,
-                                      static_cast< sweep_params * >( x.params ) );
+  k_sweep_setup<<< 1, 256, 0, x.s >>>( x.partial, kAxisBlocks, x.na + x.nb, axis, x.asc, x.bsc,
+                                       static_cast< sweep_params * >( x.params ) );
   return cudaGetLastError();
 }
 
-cudaError_t launch_sweep_keys(const sweep_launch &x) { return sweep_phase( x, true ); }
-cudaError_t launch_sweep(const sweep_launch &x) { return sweep_phase( x, false ); }
+cudaError_t launch_sweep_keys(const sweep_launch &x)
+{
+  const unsigned grid = static_cast< unsigned >( ( x.nb + kSweepThreads - 1 ) / kSweepThreads );
+  k_sweep_keys<<< grid, kSweepThreads, 0, x.s >>>( x.bverts, static_cast< int >( x.bV ), x.nb, x.eps,
+                                                   static_cast< const sweep_params * >( x.params ), x.keys, x.hist,
+                                                   static_cast< sweep_params * >( x.params ) );
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sweep(const sweep_launch &x)
+{
+  switch ( x.K )
+  {
+    case 6: return sweep_k< 6 >( x );
+    case 18: return sweep_k< 18 >( x );
+    case 26: return sweep_k< 26 >( x );
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 }  // namespace bvhg

@@ -139,13 +139,14 @@ BVHG_API bvhg_status bvhg_broadphase(bvhg_ctx *ctx, int32_t obj_a, int32_t obj_b
 BVHG_API bvhg_status bvhg_self_collision(bvhg_ctx *ctx, int32_t obj, uint64_t *pairs, uint64_t capacity, uint64_t *count,
                                 int32_t mem);
 
-/* Sort-and-sweep between two built objects (sort_and_sweep_local, src/bvh/narrowphase/kokkos.hpp:164-248): B's
- * slab minima on one cardinal axis become u32 keys over the union of both objects' extents there, a stable sort
- * orders them, and every element of A sweeps B in key order, emitting the elements that overlap it strictly on
- * every slab. axis = 0, 1 or 2, or -1 for the axis of largest centroid variance over both objects
+/* Sort-and-sweep between two built objects (sort_and_sweep_local, src/bvh/narrowphase/kokkos.hpp:164-248): B is
+ * sorted by its slab minima on one cardinal axis, cut into strips over the union of both objects' extents there and
+ * ordered within a strip by a second axis, and every element of A sweeps the strips that it can meet, emitting the
+ * elements that overlap it strictly on every slab. axis = 0, 1 or 2, or -1 for the axis of largest centroid variance
+ * over both objects
  * (max_variant_axis, kokkos.hpp:125-160); *axis_used (may be NULL) receives the axis swept. The pair set is the
  * exact S(A, B), the same as bvhg_broadphase's, for any axis (pairs as there: gid in obj_a, gid in obj_b); its
- * cost grows with the elements of B whose extents on the axis meet each element of A, so it suits patch-sized
+ * cost grows with the elements of B whose extents on the two axes come near each element of A, so it suits patch-sized
  * objects. FP64 slabs in both precision forms. obj_a != obj_b. Both objects must have been rebuilt (BVHG_REBUILD)
  * since their last bvhg_set_elements: the range and the axis come from a rebuild's bounds and centroids, which a
  * refit does not recompute (BVHG_ERR_STATE otherwise). Blocks until the count is known. */
