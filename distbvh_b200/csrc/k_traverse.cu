@@ -3,20 +3,19 @@
 // The reference finds pairs with a 4-way simultaneous recursion over two trees (get_overlapping_indices,
 // src/bvh/collision_query.hpp:293-329) or a per-entity descent (query_tree, collision_query.hpp:166-213), both
 // pruning on the strict all-slab overlap (kdop.hpp:120-125, 538-549). Here a warp walks the other object's tree
-// for a packet of 32 consecutive query ranks (Morton order: spatially coherent), one query per lane, with a stack
-// of (node, lane mask) entries: both children of a node are tested from one row holding their slabs (one 32-byte
-// FP64 / 16-byte FP32 sector per slab, loaded a chunk of slabs at a time), and a child is entered with the mask of
-// the lanes that overlap it. At a leaf bucket each lane of the mask tests its query against the bucket's
-// elements. Overlaps are emitted as (query element, tree element) local indices: through one warp-aggregated
-// reservation per bucket visit in sparse contact, through a per-warp buffer in shared memory in dense contact;
-// pairs beyond capacity are counted but not stored, so the host can grow the buffer and retry. In sparse contact
-// the grid is persistent and culls 32 packets per warp step against the target root before walking the
-// survivors; in dense contact it is one warp per packet. The FP64 recheck of the precision form reads both
-// elements' vertices per candidate and decides the overlap by comparison-only projections (kdop_math.cuh).
+// for a packet of 32 consecutive query ranks (Morton order: spatially coherent) by the packet's union box, filters the
+// elements of the buckets that it reaches, and tests those against the packet's queries (see "the walk of one
+// packet"). Overlaps are emitted as (query element, tree element) local indices through a per-warp buffer in shared
+// memory; pairs beyond capacity are counted but not stored, so the host can grow the buffer and retry. In sparse
+// contact the grid is persistent, culls 32 packets per warp step against the target root before walking the
+// survivors, and computes the element slabs it tests; in dense contact it is one warp per packet, and the element
+// slabs are stored. The FP64 recheck of the precision form reads both elements' vertices per candidate and decides
+// the overlap by comparison-only projections (kdop_math.cuh).
 //
 // Self-collision (self_collision_set, collision_query.hpp:331-368): the query of rank i only visits subtrees
 // holding ranks > i (internal node k splits its bucket range [l, r] into [l, k] and [k + 1, r]) and tests only
 // bucket elements of rank > i, so every unordered pair is found once and no element is paired with itself.
+#include <atomic>
 #include <cstddef>
 
 #include "bulk_copy.cuh"
@@ -27,102 +26,38 @@ namespace bvhg {
 int device_sm_count();
 namespace {
 
-constexpr int kTravThreads = 128;
-constexpr int kStack = 96;  // radix tree over 96-bit (key, rank) pairs: at most 95 internal levels
+// Two warps per block: a block's shared memory is free for the next one when its slower walk ends (4 warps per block:
+// the dense walks 4-5% slower).
+constexpr int kTravThreads = 64;
 
-template< typename T >
-struct slab_pair;
+// Resident blocks per SM of the walk that computes the element slabs it tests (128 registers).
+constexpr int kTravBlocksPerSM = 4 * 128 / kTravThreads;
 
-// Both children's (min, max) of one slab.
-template<>
-struct slab_pair< double >
-{
-  double min0, max0, min1, max1;
-  __device__ static slab_pair load(const double *p)
-  {
-    const double2 a = __ldg( reinterpret_cast< const double2 * >( p ) );
-    const double2 b = __ldg( reinterpret_cast< const double2 * >( p ) + 1 );
-    return { a.x, a.y, b.x, b.y };
-  }
-};
-
-template<>
-struct slab_pair< float >
-{
-  float min0, max0, min1, max1;
-  __device__ static slab_pair load(const float *p)
-  {
-    const float4 a = __ldg( reinterpret_cast< const float4 * >( p ) );
-    return { a.x, a.y, a.z, a.w };
-  }
-};
-
-// Axes of a node row loaded together in the walk (a chunk of loads in flight per round trip; bounded by registers).
-template< int K, typename T >
-constexpr int kNodeChunk = ( K / 2 ) <= 4 ? K / 2 : ( sizeof( T ) == 4 ? ( K / 2 + 1 ) / 2 : 5 );
-
-// Resident blocks per SM of the single-node walk, which computes the element slabs it tests (128 registers).
-constexpr int kTravBlocksPerSM = 4;
-
-// Slots for k outputs of each calling lane, one atomic per group of converged lanes: the lanes' exclusive prefix of
-// k is formed from one ballot per bit of k (k < 64), the lowest lane reserves the group's total.
-__device__ __forceinline__ unsigned long long warp_reserve(unsigned k, unsigned long long *counter)
-{
-  const unsigned active = __activemask();
-  const unsigned lane = threadIdx.x & 31u;
-  const unsigned lt = ( 1u << lane ) - 1u;
-  unsigned pre = 0, tot = 0;
-#pragma unroll
-  for ( int bit = 0; bit < 6; ++bit )
-  {
-    const unsigned bal = __ballot_sync( active, ( k >> bit ) & 1u );
-    pre += static_cast< unsigned >( __popc( bal & lt ) ) << bit;
-    tot += static_cast< unsigned >( __popc( bal ) ) << bit;
-  }
-  const int leader = __ffs( active ) - 1;
-  unsigned long long base = 0;
-  if ( static_cast< int >( lane ) == leader && tot ) base = atomicAdd( counter, static_cast< unsigned long long >( tot ) );
-  base = __shfl_sync( active, base, leader );
-  return base + pre;
-}
-
-// Slabs of element e straight into a shared-memory row (C = 2 D values: min, max per slab): the same FP64 slabs
-// (slab by slab, so that only the vertices stay in registers), or the same FP32 enclosures, that slabs_body
-// unites into the bucket boxes.
+// Slabs of element e straight into a shared-memory row (K values: min, max per slab): the same FP64 slabs (slab by
+// slab, so that only the vertices stay in registers), or the same FP32 enclosures, that slabs_body unites into the
+// bucket boxes.
 template< int K, typename T, int VT >
 __device__ __forceinline__ void slabs_to_row(const double *__restrict__ verts, uint32_t Vrt, uint32_t e, double eps,
                                              float eps_hi, T *row)
 {
   constexpr int D = K / 2;
-  if constexpr ( VT > 0 )
+  if constexpr ( VT > 0 && sizeof( T ) == 8 )
   {
     double p[VT * 3];
     const double *src = verts + static_cast< size_t >( e ) * VT * 3;
 #pragma unroll
     for ( int k = 0; k < VT * 3; ++k ) p[k] = __ldg( src + k );
-    if constexpr ( sizeof( T ) == 8 )
+#pragma unroll
+    for ( int a = 0; a < D; ++a )
     {
-#pragma unroll
-      for ( int a = 0; a < D; ++a )
-      {
-        double l, h;
-        slab64< K >( p, VT, a, eps, l, h );
-        row[2 * a] = l;
-        row[2 * a + 1] = h;
-      }
-    } else {
-      float lo[D], hi[D];
-      slabs32_all< K, VT >( p, eps_hi, lo, hi );
-#pragma unroll
-      for ( int a = 0; a < D; ++a )
-      {
-        row[2 * a] = lo[a];
-        row[2 * a + 1] = hi[a];
-      }
+      double l, h;
+      slab64< K >( p, VT, a, eps, l, h );
+      row[2 * a] = l;
+      row[2 * a + 1] = h;
     }
   } else {
     T lo[D], hi[D];
-    leaf_slabs< K, T, 0 >( verts, Vrt, e, eps, eps_hi, lo, hi );
+    leaf_slabs< K, T, VT >( verts, Vrt, e, eps, eps_hi, lo, hi );
 #pragma unroll
     for ( int a = 0; a < D; ++a )
     {
@@ -132,14 +67,22 @@ __device__ __forceinline__ void slabs_to_row(const double *__restrict__ verts, u
   }
 }
 
-// Everything one query packet needs besides the tree (see traverse_body).
+// The three cardinal slabs of element e, as leaf_slabs forms them.
+template< int K, typename T, int VT >
+__device__ __forceinline__ void cardinal_slabs(const double *__restrict__ verts, uint32_t Vrt, uint32_t e, double eps,
+                                               float eps_hi, T *lo, T *hi)
+{
+  leaf_slabs< 6, T, VT >( verts, Vrt, e, eps, eps_hi, lo, hi );
+}
+
+// Everything one query packet needs besides the tree (see walk_packet).
 template< typename T >
 struct trav_args
 {
   const T *qwarp;
   const double *qverts;
   uint32_t qV;
-  const T *qrows;    // query element slabs in rank order (stored variant only)
+  const T *qrows;    // query element slabs in rank order (stored form only)
   const uint32_t *qperm;
   uint32_t nq;
   const int2 *child;
@@ -147,7 +90,7 @@ struct trav_args
   const int2 *range;
   const double *tverts;
   uint32_t tV;
-  const T *tcache;   // element slabs of the target in rank order (stored variant only)
+  const T *tcache;   // element slabs of the target in rank order (stored form only)
   const uint32_t *tperm;
   const obj_scalars *tsc;
   uint32_t nt;
@@ -157,7 +100,7 @@ struct trav_args
   uint2 *pairs;
   uint64_t cap;
   pair_scalars *ps;
-  int dense_stack;  // stack bound of the batched dense walk (kDenseStack, lower under a test hook)
+  int stack_limit;  // stack bound of the walk over stored slabs (kWalkStack, lower under a test hook)
 };
 
 // The typed view of a scene's traversal item.
@@ -186,250 +129,83 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
   x.pairs = it.pairs;
   x.cap = it.cap;
   x.ps = it.ps;
-  x.dense_stack = it.dense_stack;
+  x.stack_limit = it.dense_stack;
   return x;
 }
 
-// Target leaf bucket bb for the lanes in `mine`: the warp first computes the bucket's element slabs into its cache
-// (lane j: element of rank 8 bb + j), then every lane of the mask tests its query against them (ranks above its own
-// in self-collision). Hits go out through one warp-aggregated reservation. Called by the whole warp.
-template< int K, typename T, int VT >
-__device__ __forceinline__ void test_bucket(const trav_args< T > &x, const T *qlo, const T *qhi, uint32_t qe, int bb,
-                                            int skip, bool mine, T *cache, unsigned lane)
-{
-  constexpr int D = K / 2;
-  const int t0 = kLeafSize * bb;
-  const int cnt = min( kLeafSize, static_cast< int >( x.nt ) - t0 );
-  // The bucket's element slabs, computed from the vertices into the warp's shared-memory cache by lanes 0..7
-  // (sparse contact: a bucket is tested by few packets, so nothing is kept).
-  if ( static_cast< int >( lane ) < cnt )
-    slabs_to_row< K, T, VT >( x.tverts, x.tV, __ldg( x.tperm + t0 + lane ), x.eps, x.eps_hi, cache + lane * 2 * D );
-  __syncwarp();
-  const T *rows = cache;
-  if ( mine )
-  {
-    const int r0 = max( t0, skip + 1 );
-    unsigned hits = 0;
-    for ( int r = r0; r < t0 + cnt; ++r )
-    {
-      const T *eb = rows + ( r - t0 ) * 2 * D;
-      bool o = true;
-#pragma unroll
-      for ( int a = 0; a < D; ++a )
-      {
-        if ( !o ) break;
-        o = qlo[a] < eb[2 * a + 1] && eb[2 * a] < qhi[a];
-      }
-      if ( o ) hits |= 1u << ( r - t0 );
-    }
-    unsigned long long pos = warp_reserve( static_cast< unsigned >( __popc( hits ) ), &x.ps->count );
-    for ( ; hits; hits &= hits - 1, ++pos )
-      if ( pos < x.cap ) x.pairs[pos] = make_uint2( qe, __ldg( x.tperm + t0 + __ffs( hits ) - 1 ) );
-  }
-  __syncwarp();  // the cache is refilled by the next leaf
-}
-
-// One packet: the union box of ranks pk*32 .. pk*32 + 31 against the target root, then the walk (see traverse_body).
-template< int K, typename T, int VT >
-__device__ __forceinline__ void traverse_packet(const trav_args< T > &x, const uint32_t i, const unsigned lane,
-                                                int2 *stack, T *cache, const T *rb)
-{
-  constexpr int D = K / 2;
-  constexpr int D0 = D < 4 ? D : 4;
-  // 1. The packet's union box against the target's root box, first four slabs first (uniform per warp).
-  {
-    const T *wb = x.qwarp + static_cast< size_t >( i >> 5 ) * D * 2;
-    bool o = true;
-#pragma unroll
-    for ( int a = 0; a < D0; ++a ) o = o && ( __ldg( wb + 2 * a ) < rb[2 * a + 1] && rb[2 * a] < __ldg( wb + 2 * a + 1 ) );
-    if ( !o ) return;
-#pragma unroll
-    for ( int a = D0; a < D; ++a ) o = o && ( __ldg( wb + 2 * a ) < rb[2 * a + 1] && rb[2 * a] < __ldg( wb + 2 * a + 1 ) );
-    if ( !o ) return;
-  }
-  // 2. Each lane's own slabs, from its element's vertices, against the root box.
-  const bool valid = i < x.nq;
-  const uint32_t qe = valid ? __ldg( x.qperm + i ) : 0u;
-  T qlo[D], qhi[D];
-  bool in_root = valid;
-  if ( valid ) leaf_slabs< K, T, VT >( x.qverts, x.qV, qe, x.eps, x.eps_hi, qlo, qhi );
-#pragma unroll
-  for ( int a = 0; a < D; ++a )
-  {
-    if ( !valid )
-    {
-      qlo[a] = T( 0 );
-      qhi[a] = T( 0 );
-    }
-    in_root = in_root && ( qlo[a] < rb[2 * a + 1] && rb[2 * a] < qhi[a] );
-  }
-  unsigned mask = __ballot_sync( 0xffffffffu, in_root );
-  if ( !mask ) return;
-  const int skip = x.self ? static_cast< int >( i ) : -1;  // self-collision: only ranks above the query's
-  const int root = x.tsc->root;
-  if ( root < 0 )
-  {
-    test_bucket< K, T, VT >( x, qlo, qhi, qe, ~root, skip, in_root, cache, lane );
-    return;
-  }
-  int sp = 0;
-  int node = root;
-  while ( true )
-  {
-    const bool me = ( mask >> lane ) & 1u;
-    const int2 c = __ldg( x.child + node );
-    const T *nb = x.nbox + static_cast< size_t >( node ) * D * 4;
-    bool o0 = me, o1 = me;
-    if ( x.self )
-    {
-      // left child covers buckets [l, node], right child [node + 1, r]; skip subtrees whose last rank <= i
-      o0 = o0 && kLeafSize * node + kLeafSize - 1 > static_cast< int >( i );
-      o1 = o1 && min( kLeafSize * __ldg( &x.range[node].y ) + kLeafSize - 1, static_cast< int >( x.nt ) - 1 ) >
-                   static_cast< int >( i );
-    }
-    // The node row's slabs in chunks of kNodeChunk axes: a chunk's loads (one sector per axis) are all in flight
-    // before its tests, and the warp stops between chunks once no lane overlaps either child.
-#pragma unroll
-    for ( int a0 = 0; a0 < D; a0 += kNodeChunk< K, T > )
-    {
-      if ( a0 > 0 && !__any_sync( 0xffffffffu, o0 || o1 ) ) break;
-      slab_pair< T > sl[kNodeChunk< K, T >];
-#pragma unroll
-      for ( int j = 0; j < kNodeChunk< K, T >; ++j )
-        if ( a0 + j < D ) sl[j] = slab_pair< T >::load( nb + ( a0 + j ) * 4 );
-#pragma unroll
-      for ( int j = 0; j < kNodeChunk< K, T >; ++j )
-      {
-        if ( a0 + j >= D ) break;
-        o0 = o0 && ( qlo[a0 + j] < sl[j].max0 && sl[j].min0 < qhi[a0 + j] );
-        o1 = o1 && ( qlo[a0 + j] < sl[j].max1 && sl[j].min1 < qhi[a0 + j] );
-      }
-    }
-    const unsigned m0 = __ballot_sync( 0xffffffffu, o0 );
-    const unsigned m1 = __ballot_sync( 0xffffffffu, o1 );
-    int next = -1;
-    unsigned nmask = 0;
-    if ( m0 )
-    {
-      if ( c.x < 0 ) test_bucket< K, T, VT >( x, qlo, qhi, qe, ~c.x, skip, o0, cache, lane );
-      else
-      {
-        next = c.x;
-        nmask = m0;
-      }
-    }
-    if ( m1 )
-    {
-      if ( c.y < 0 ) test_bucket< K, T, VT >( x, qlo, qhi, qe, ~c.y, skip, o1, cache, lane );
-      else if ( next < 0 )
-      {
-        next = c.y;
-        nmask = m1;
-      } else {
-        if ( sp == kStack )
-        {
-          if ( lane == 0 ) atomicCAS( &x.ps->error, 0, kErrOverflowStack );
-          return;
-        }
-        if ( lane == 0 ) stack[sp] = make_int2( c.y, static_cast< int >( m1 ) );
-        ++sp;
-      }
-    }
-    if ( next < 0 )
-    {
-      if ( sp == 0 ) break;
-      __syncwarp();
-      const int2 e = stack[--sp];
-      next = e.x;
-      nmask = static_cast< unsigned >( e.y );
-    }
-    __syncwarp();
-    node = next;
-    mask = nmask;
-  }
-}
-
-// One warp per group of 32 query ranks (a packet), lane = query element. The warp walks the target tree once for
-// its packet: every lane tests its own element's slabs (computed from its vertices) against both children of the
-// current node (the node row is read once for the warp, a broadcast), and a child is entered with the mask of the
-// lanes that overlap it (a lane that misses a node misses all of its descendants). Stack entries are (node, lane
-// mask), in shared memory. At a leaf bucket the lanes of the mask test their element against the bucket's element
-// slabs, computed once by the warp from the vertices into a shared cache.
-template< int K, typename T, int VT >
-__device__ void traverse_body(const trav_item &item, uint32_t, uint32_t)
-{
-  const trav_args< T > x = typed< T >( item );
-  const obj_scalars *__restrict__ qsc = item.qsc;
-  constexpr int D = K / 2;
-  constexpr int D0 = D < 4 ? D : 4;
-  constexpr int WPB = kTravThreads / 32;
-  __shared__ int2 s_stack[WPB][kStack];                          // (node, lane mask)
-  __shared__ __align__( 16 ) T s_cache[WPB][kLeafSize * 2 * D];  // slabs of the leaf bucket being tested
-  const unsigned lane = threadIdx.x & 31u;
-  int2 *stack = s_stack[threadIdx.x >> 5];
-  T *cache = s_cache[threadIdx.x >> 5];
-  // No tree exists after a failed sort of either object.
-  if ( *reinterpret_cast< const volatile int * >( &x.tsc->error ) == kErrTimeout ||
-       *reinterpret_cast< const volatile int * >( &qsc->error ) == kErrTimeout )
-    return;
-  const T *rb = reinterpret_cast< const T * >( x.tsc->root_box );
-  // 0. Root against root: objects far apart (most pairs of a batch) end here for the whole grid.
-  {
-    const T *qr = reinterpret_cast< const T * >( qsc->root_box );
-    bool o = true;
-#pragma unroll
-    for ( int a = 0; a < D0; ++a ) o = o && ( qr[2 * a] < rb[2 * a + 1] && rb[2 * a] < qr[2 * a + 1] );
-    if ( !o ) return;
-  }
-  const uint32_t packets = ( x.nq + 31 ) / 32;
-  // Packets (32 query ranks) in a persistent grid. A warp takes chunks from the pair counters'
-  // packet dispenser; chunk c holds the packets c, c + C, c + 2C, ... (C chunks), so a contact region (consecutive
-  // Morton ranks) is spread over many chunks. Lane j tests the union box of the chunk's packet j against the target
-  // root (one load per lane for the packets far from the target), then the warp walks the survivors one after the
-  // other.
-  const uint32_t chunks = ( packets + 31 ) / 32;
-  while ( true )
-  {
-    uint32_t c = 0;
-    if ( lane == 0 ) c = atomicAdd( &x.ps->packet_next, 1u );
-    c = __shfl_sync( 0xffffffffu, c, 0 );
-    if ( c >= chunks ) break;
-    const uint64_t pk = c + static_cast< uint64_t >( lane ) * chunks;
-    bool o = false;
-    if ( pk < packets )
-    {
-      const T *wb = x.qwarp + pk * D * 2;
-      o = true;
-#pragma unroll
-      for ( int a = 0; a < D; ++a ) o = o && ( __ldg( wb + 2 * a ) < rb[2 * a + 1] && rb[2 * a] < __ldg( wb + 2 * a + 1 ) );
-    }
-    for ( unsigned m = __ballot_sync( 0xffffffffu, o ); m; m &= m - 1 )
-    {
-      const uint32_t p = c + static_cast< uint32_t >( __ffs( m ) - 1 ) * chunks;
-      traverse_packet< K, T, VT >( x, p * 32 + lane, lane, stack, cache, rb );
-    }
-  }
-}
-
-// ---- dense contact: both objects' element slabs stored ----------------------------------------------------------
+// ---- the walk of one packet -----------------------------------------------------------------------------------
 //
-// In dense contact a packet's walk visits a few hundred internal nodes and tens of leaf buckets, each shared by only
-// a fraction of the packet's 32 queries. Two changes over the walk of traverse_packet:
-//   - Nodes in batches. Each step pops up to kDenseBatch (4 or 6) (node, lane mask) entries from the stack; the
-//     warp copies their rows (both children's slabs) into shared memory with one round of 16-byte asynchronous
-//     copies, and every lane tests its query against the children of each popped node whose mask holds it, from
-//     shared memory. One global round trip serves the whole batch instead of one per chunk of slabs per node.
-//   - Leaves in batches. The walk only queues (bucket, lane mask) entries; a flush spreads all (query, element)
-//     tests of the queued entries over the warp's lanes, 32 at a time, with every query's slabs staged in shared
-//     memory and the target elements' stored rows read from global memory. A lane finds the entry of its test from
-//     two warp votes per round and reads it from the lane that holds it. Hits collect in a per-warp buffer in
-//     shared memory (one ballot per 32 tests); a full buffer leaves through one atomic reservation and coalesced
-//     stores, so a warp pays an atomic's round trip per 33-64 pairs instead of per round of tests with a hit.
-// The stack grows by at most kDenseBatch entries per step, so its depth bound is kDenseStack; a walk that would pass
-// it raises kErrOverflowStack, and the host then runs the pair search again with the single-node walk (whose stack
-// is bounded by the tree depth).
-constexpr int kLeafQueue = 32;  // queued (bucket, mask) entries per warp
+// A packet is 32 consecutive query ranks and belongs to one warp. Its walk has five kinds of steps, each with its own
+// use of the lanes:
+//   - Expand: lane = (node, child). Up to 16 nodes are popped from the packet's stack; every lane tests one child's
+//     slabs against the packet's union box. A leaf bucket that passes goes onto the bucket list, an internal node back
+//     onto the stack; children smaller than half the packet's box go onto the check list first.
+//   - Check: lane = query. The cardinal slabs of the listed boxes are staged in shared memory, eight boxes at a time,
+//     and every lane tests its query against them. A child that no query overlaps is dropped.
+//   - Filter: lane = element of four listed buckets. The elements that overlap the packet's union box are gathered, 16
+//     at a time, as rows in shared memory.
+//   - Cardinal tests: lane = (query of two, gathered element), the element's cardinal slabs in registers, over the
+//     packet's queries. Survivors collect in a list in shared memory.
+//   - Slab tests: lane = survivor (query, element), on the other slabs.
+// Everything larger than a query costs one lane-test per box or element instead of 32. On a tet lattice at 26-DOP a
+// packet meets 157 nodes, 49 buckets of 390 elements, 149 elements that overlap its box, 310 survivors and 133 pairs
+// (counted on the host over 64^3 cells). A walk of (node, lane mask) entries that tests all 32 queries against every
+// node, and every query against every element of the buckets that it overlaps, makes 175 x 64 box tests and 1455
+// element tests on all slabs for them, most on idle lanes.
+// What bounds it is the chain of dependent reads and the instructions per test, so a step reads all slabs of its nodes
+// or elements at once (one trip to memory per step) and compares without branches.
+// Traversal of the 256^3 lattice at 26-DOP FP64 25.6 -> 13.9 ms; 161^3 at 18-DOP FP32 2.53 -> 1.46 ms; 200,003
+// tetrahedra against themselves 208 -> 151 us; two plates of 10,000 triangles 186 -> 91 us; in sparse contact the
+// sphere on the plate (9.4M triangles) 105 -> 63 us. Measured and slower: the same expansion, then all 32 queries
+// against every bucket and four queries by eight elements per round from shared memory (15.4 ms); the same with a
+// second round for the non-cardinal slabs by (survivor, slab) lanes (29 ms); rows read five slabs at a time (20 to 50
+// ms, depending on the resident warps).
+// A packet whose ranks straddle a jump of the Morton curve, or whose elements lie far apart, has a union box that says
+// little: the check of the small children keeps its walk on the nodes that one of its queries overlaps.
+//
+// The element slabs come from the rows that the slab kernel stored (STORED: dense contact; slab-major per bucket, so
+// that the filter reads the pairs of one slab of eight elements as one piece) or are computed from the vertices: the
+// packet's 32 queries once, and the gathered elements (there the filter tests the cardinal slabs only).
+//
+// Stack bound: the wide steps stop while stack and list hold more than stack_limit - 32 - kWalkDepth entries; the walk
+// then expands one node at a time and checks the list after each, which is a depth-first walk and adds at most one
+// entry per tree level (at most 95). kWalkStack entries therefore always suffice. A lower stack_limit (test hook) can
+// be reached: the walk raises kErrOverflowStack, and the host runs the pair search again with computed slabs.
+constexpr int kWalkDepth = 96;  // radix tree over 96-bit (key, rank) pairs: at most 95 internal levels
+constexpr int kWalkStack = 288;
+constexpr int kCheckCap = 64;   // listed children: checked once more than 32 are held
+constexpr int kCheckRows = 8;   // boxes staged per check step
+constexpr int kLeafCap = 64;    // listed buckets: filtered once more than 32 are held
+constexpr int kGather = 16;     // elements gathered before they are tested
+constexpr int kSurvivors = 128;  // (query, element) pairs past the cardinal tests: tested once 32 are held
 constexpr int kPairBuf = 64;    // buffered pairs per warp: drained once more than 32 are held
+
+template< int K, typename T >
+struct walk_smem
+{
+  // read as (min, max) pairs, and written by asynchronous copies of pairs
+  alignas( 16 ) T q[32][K];             // slabs of the packet's queries
+  alignas( 16 ) T e[kGather][K];        // slabs of the gathered elements
+  alignas( 16 ) T rows[kCheckRows][6];  // cardinal slabs of the boxes being checked
+  alignas( 16 ) T g[K];                 // the packet's union box
+  alignas( 16 ) uint2 out[kPairBuf];    // pairs found and not yet written
+  int2 list[kCheckCap];                 // (2 * parent + side, child link) to check
+  int leaf[kLeafCap];                   // buckets to filter
+  int stack[kWalkStack];                // internal nodes to expand
+  uint32_t qe[32];                      // query element indices
+  uint32_t te[kGather], tr[kGather];    // element indices and ranks of the gathered elements
+  uint16_t surv[kSurvivors];            // query | gathered element << 8
+};
+
+// The state of a warp's walk.
+struct walk_state
+{
+  uint32_t i0;    // first query rank of the packet
+  unsigned lane;
+  unsigned in;    // queries that overlap the target's root box
+  int ne = 0;     // gathered elements
+  uint32_t ns = 0, nout = 0;
+};
 
 // A (min, max) pair: from global memory (read-only path) or from shared memory, as one vector load.
 __device__ __forceinline__ void load_pair(const double *p, double &lo, double &hi)
@@ -456,328 +232,456 @@ __device__ __forceinline__ void shared_pair(const float *p, float &lo, float &hi
   lo = v.x;
   hi = v.y;
 }
-// Nodes popped per step: 6 for 26-DOP FP64 rows (measured 6% faster there, at 4 resident blocks per SM instead of
-// 5), 4 otherwise (6 measured 1-6% slower for the other k-DOPs and the FP32 rows).
-template< int K, typename T >
-constexpr int kDenseBatch = ( K == 26 && sizeof( T ) == 8 ) ? 6 : 4;
-constexpr int kDenseStack = 256;
-
-template< int K, typename T >
-struct dense_smem
-{
-  // every array starts on a 16-byte boundary: rows[] receives 16-byte asynchronous copies, and q[] and rows[] are
-  // read as 8- or 16-byte (min, max) pairs
-  alignas( 16 ) T q[32][K];                  // query slabs of the packet, (min, max) per slab
-  alignas( 16 ) T rows[kDenseBatch< K, T >][2 * K];  // node rows of the batch: [slab][child][min, max]
-  alignas( 16 ) uint32_t qe[32];             // query element indices
-  alignas( 16 ) int2 stack[kDenseStack];     // (node, lane mask)
-  alignas( 16 ) int2 leaf[kLeafQueue];       // (bucket, lane mask)
-  alignas( 16 ) uint2 out[kPairBuf];         // pairs found and not yet written
-};
-
-template< int K, typename T >
-constexpr bool dense_smem_aligned()
-{
-  using S = dense_smem< K, T >;
-  return offsetof( S, q ) % 16 == 0 && offsetof( S, rows ) % 16 == 0 && sizeof( S ) % 16 == 0 &&
-         ( 2 * K * sizeof( T ) ) % 16 == 0;  // node rows: whole 16-byte pieces
-}
-static_assert( dense_smem_aligned< 6, double >() && dense_smem_aligned< 18, double >() &&
-                 dense_smem_aligned< 26, double >() && dense_smem_aligned< 6, float >() &&
-                 dense_smem_aligned< 18, float >() && dense_smem_aligned< 26, float >(),
-               "dense walk shared memory must keep 16-byte alignment" );
+__device__ __forceinline__ void copy_pair(double *dst, const double *src) { cp_async16( dst, src ); }
+__device__ __forceinline__ void copy_pair(float *dst, const float *src) { cp_async_small< 8 >( dst, src ); }
 
 // Writes the warp's buffered pairs: one atomic reservation for all of them, then coalesced stores (a count past
 // the capacity is still counted, so the host learns the size it needs).
 template< int K, typename T >
-__device__ __forceinline__ void drain_pairs(const trav_args< T > &x, dense_smem< K, T > &sm, uint32_t &nout,
-                                            unsigned lane)
+__device__ __forceinline__ void drain_pairs(const trav_args< T > &x, walk_smem< K, T > &sm, walk_state &w)
 {
   __syncwarp();
   unsigned long long base = 0;
-  if ( lane == 0 && nout ) base = atomicAdd( &x.ps->count, static_cast< unsigned long long >( nout ) );
+  if ( w.lane == 0 && w.nout ) base = atomicAdd( &x.ps->count, static_cast< unsigned long long >( w.nout ) );
   base = __shfl_sync( 0xffffffffu, base, 0 );
-  for ( uint32_t j = lane; j < nout; j += 32 )
+  for ( uint32_t j = w.lane; j < w.nout; j += 32 )
     if ( base + j < x.cap ) x.pairs[base + j] = sm.out[j];
   __syncwarp();
-  nout = 0;
+  w.nout = 0;
 }
 
-// Tests every (query, element) pair of the queued entries; i0 = the packet's first query rank. Hits are appended to
-// the warp's pair buffer (nout pairs held).
+// Appends the pairs (q, e) of the lanes with hit.
 template< int K, typename T >
-__device__ __forceinline__ void flush_leaves(const trav_args< T > &x, dense_smem< K, T > &sm, int nleaf, uint32_t i0,
-                                             unsigned lane, uint32_t &nout)
+__device__ __forceinline__ void emit(const trav_args< T > &x, walk_smem< K, T > &sm, walk_state &w, bool hit, uint32_t q, uint32_t e)
+{
+  const unsigned m = __ballot_sync( 0xffffffffu, hit );
+  if ( !m ) return;
+  if ( hit ) sm.out[w.nout + __popc( m & ( ( 1u << w.lane ) - 1u ) )] = make_uint2( sm.qe[q], sm.te[e] );
+  w.nout += static_cast< uint32_t >( __popc( m ) );
+  if ( w.nout > kPairBuf - 32 ) drain_pairs( x, sm, w );
+}
+
+// The slab tests of `count` (at most 32) listed survivors from `first` on.
+template< int K, typename T >
+__device__ __forceinline__ void test_survivors(const trav_args< T > &x, walk_smem< K, T > &sm, walk_state &w, uint32_t first,
+                                               uint32_t count)
 {
   constexpr int D = K / 2;
-  __syncwarp();
-  const int2 ent = static_cast< int >( lane ) < nleaf ? sm.leaf[lane] : make_int2( 0, 0 );
-  const uint32_t c = 8u * static_cast< uint32_t >( __popc( static_cast< unsigned >( ent.y ) ) );
-  uint32_t inc = c;
+  const bool act = w.lane < count;
+  const uint32_t s = act ? sm.surv[first + w.lane] : 0u, q = s & 31u, e = s >> 8;
+  const T *qr = sm.q[q], *er = sm.e[e];
+  bool lo_ok = act, hi_ok = true;  // bitwise: no branch per comparison
 #pragma unroll
-  for ( int o = 1; o < 32; o <<= 1 )
+  for ( int a = 3; a < D; ++a )
   {
-    const uint32_t y = __shfl_up_sync( 0xffffffffu, inc, o );
-    if ( lane >= static_cast< unsigned >( o ) ) inc += y;
+    T ql, qh, el, eh;
+    shared_pair( qr + 2 * a, ql, qh );
+    shared_pair( er + 2 * a, el, eh );
+    lo_ok &= ql < eh;
+    hi_ok &= el < qh;
   }
-  const uint32_t total = __shfl_sync( 0xffffffffu, inc, 31 );
-  const bool is_entry = static_cast< int >( lane ) < nleaf;
-  const uint32_t mypre = inc - c;
+  emit( x, sm, w, lo_ok & hi_ok, q, e );
+}
+
+// All tests of the gathered elements; leaves none. Half a warp takes one query each round (two rounds in flight).
+template< int K, typename T >
+__device__ __forceinline__ void test_gathered(const trav_args< T > &x, walk_smem< K, T > &sm, walk_state &w)
+{
+  cp_async_wait_all();
   __syncwarp();
-  const unsigned lt = ( 1u << lane ) - 1u;
-  for ( uint32_t base = 0; base < total; base += 32 )
+  const uint32_t e = w.lane & ( kGather - 1u );
+  const bool act = static_cast< int >( e ) < w.ne, upper = w.lane >= kGather;
+  T el[3], eh[3];
+#pragma unroll
+  for ( int a = 0; a < 3; ++a ) shared_pair( &sm.e[e][2 * a], el[a], eh[a] );
+  // self-collision: only the queries of lower rank
+  const uint32_t above = act ? ( x.self ? sm.tr[e] - w.i0 : 32u ) : 0u;
+  constexpr int U = 2;
+  for ( unsigned m = w.in; m; )
   {
-    const uint32_t g = base + lane;
-    bool hit = false;
-    uint32_t q = 0, r = 0;
-    // the entry of test g: the last entry whose prefix is <= g, from the entries that start before this round and
-    // the starts inside it (entries have distinct prefixes: every entry holds at least 8 tests)
-    const unsigned before = __ballot_sync( 0xffffffffu, is_entry && mypre < base );
-    const unsigned inround = ( is_entry && mypre >= base && mypre - base < 32u ) ? ( 1u << ( mypre - base ) ) : 0u;
-    const unsigned starts = __reduce_or_sync( 0xffffffffu, inround );
-    int lo = __popc( before ) + __popc( starts & ( ( 2u << lane ) - 1u ) ) - 1;
-    lo = lo < 0 ? 0 : lo;
-    const uint32_t lpre = __shfl_sync( 0xffffffffu, mypre, lo );
-    const int enx = __shfl_sync( 0xffffffffu, ent.x, lo ), eny = __shfl_sync( 0xffffffffu, ent.y, lo );
-    if ( g < total )
+    uint32_t q[U];
+    bool ok[U];
+#pragma unroll
+    for ( int u = 0; u < U; ++u )
     {
-      const uint32_t rr = g - lpre;
-      const int2 en = make_int2( enx, eny );
-      unsigned m = static_cast< unsigned >( en.y );
-      for ( uint32_t k = rr >> 3; k > 0; --k ) m &= m - 1;  // the (rr / 8)-th query of the entry's mask
-      q = static_cast< uint32_t >( __ffs( m ) - 1 );
-      r = static_cast< uint32_t >( en.x ) * kLeafSize + ( rr & 7u );
-      if ( r < x.nt && ( !x.self || r > i0 + q ) )
+      const unsigned rest = m & ( m - 1u );
+      const unsigned mine = upper ? rest : m;
+      ok[u] = mine != 0u;
+      q[u] = mine ? static_cast< uint32_t >( __ffs( mine ) - 1 ) : 0u;
+      m = rest & ( rest - 1u );
+      ok[u] &= q[u] < above;
+      const T *qr = sm.q[q[u]];
+#pragma unroll
+      for ( int a = 0; a < 3; ++a )
       {
-        // a chunk of slabs of the element (global) and of the query (shared) is loaded before it is tested
-        const T *er = x.tcache + static_cast< size_t >( r >> 3 ) * ( kLeafSize * K ) + 2 * ( r & 7u );
-        const T *qr = sm.q[q];
-        hit = true;
-#pragma unroll
-        for ( int a0 = 0; a0 < D; a0 += kNodeChunk< K, T > )
-        {
-          if ( !hit ) break;
-          T ev[2 * kNodeChunk< K, T >], qv[2 * kNodeChunk< K, T >];
-#pragma unroll
-          for ( int j = 0; j < kNodeChunk< K, T >; ++j )
-          {
-            if ( a0 + j >= D ) break;
-            load_pair( er + 2 * kLeafSize * ( a0 + j ), ev[2 * j], ev[2 * j + 1] );
-            shared_pair( qr + 2 * ( a0 + j ), qv[2 * j], qv[2 * j + 1] );
-          }
-#pragma unroll
-          for ( int j = 0; j < kNodeChunk< K, T >; ++j )
-          {
-            if ( a0 + j >= D ) break;
-            hit = hit && qv[2 * j] < ev[2 * j + 1] && ev[2 * j] < qv[2 * j + 1];
-          }
-        }
+        T ql, qh;
+        shared_pair( qr + 2 * a, ql, qh );
+        ok[u] &= ( ql < eh[a] ) & ( el[a] < qh );
       }
     }
-    const unsigned bal = __ballot_sync( 0xffffffffu, hit );
-    if ( bal )
+#pragma unroll
+    for ( int u = 0; u < U; ++u )
     {
-      if ( hit ) sm.out[nout + static_cast< unsigned >( __popc( bal & lt ) )] = make_uint2( sm.qe[q], __ldg( x.tperm + r ) );
-      nout += static_cast< uint32_t >( __popc( bal ) );
-      if ( nout > kPairBuf - 32 ) drain_pairs< K, T >( x, sm, nout, lane );
+      if constexpr ( K == 6 )
+      {
+        emit( x, sm, w, ok[u], q[u], e );
+      } else {
+        const unsigned bal = __ballot_sync( 0xffffffffu, ok[u] );
+        if ( ok[u] ) sm.surv[w.ns + __popc( bal & ( ( 1u << w.lane ) - 1u ) )] = static_cast< uint16_t >( q[u] | ( e << 8 ) );
+        w.ns += static_cast< uint32_t >( __popc( bal ) );
+      }
+    }
+    if constexpr ( K > 6 )
+    {
+      if ( w.ns >= 32u )
+      {
+        // the last 32 (or twice 32) are tested; the others stay where they are
+        __syncwarp();
+        do
+        {
+          w.ns -= 32u;
+          test_survivors( x, sm, w, w.ns, 32u );
+        } while ( w.ns >= 32u );
+        __syncwarp();
+      }
+    }
+  }
+  if constexpr ( K > 6 )
+  {
+    if ( w.ns )
+    {
+      __syncwarp();
+      test_survivors( x, sm, w, 0u, w.ns );
+      w.ns = 0;
+    }
+  }
+  __syncwarp();
+  w.ne = 0;
+}
+
+// The filter of the nleaf listed buckets.
+template< int K, typename T, int VT, bool STORED >
+__device__ __forceinline__ void filter_buckets(const trav_args< T > &x, walk_smem< K, T > &sm, walk_state &w, int nleaf)
+{
+  constexpr int D = K / 2;
+  for ( int b0 = 0; b0 < nleaf; b0 += 4 )
+  {
+    const int b = b0 + static_cast< int >( w.lane >> 3 );
+    const int bucket = b < nleaf ? sm.leaf[b] : 0;
+    const uint32_t r = static_cast< uint32_t >( kLeafSize * bucket ) + ( w.lane & 7u );
+    bool o = b < nleaf && r < x.nt && ( !x.self || r > w.i0 );
+    const uint32_t te = o ? __ldg( x.tperm + r ) : 0u;
+    const T *src = STORED ? x.tcache + static_cast< size_t >( bucket ) * ( kLeafSize * K ) + 2 * ( w.lane & 7u ) : nullptr;
+    bool lo_ok = true, hi_ok = true;  // bitwise: no branch per comparison
+    if ( o )
+    {
+      // all slabs at once (stored form): one trip to memory per four buckets
+      constexpr int F = STORED ? D : 3;
+      T lo[F], hi[F];
+      if constexpr ( STORED )
+      {
+#pragma unroll
+        for ( int a = 0; a < F; ++a ) load_pair( src + 2 * kLeafSize * a, lo[a], hi[a] );
+      } else {
+        cardinal_slabs< K, T, VT >( x.tverts, x.tV, te, x.eps, x.eps_hi, lo, hi );
+      }
+#pragma unroll
+      for ( int a = 0; a < F; ++a )
+      {
+        T gl, gh;
+        shared_pair( &sm.g[2 * a], gl, gh );
+        lo_ok &= gl < hi[a];
+        hi_ok &= lo[a] < gh;
+      }
+      o = lo_ok & hi_ok;
+    }
+    // the elements that passed become rows; full rows are tested
+    for ( unsigned m = __ballot_sync( 0xffffffffu, o ); m; )
+    {
+      const int at = w.ne + __popc( m & ( ( 1u << w.lane ) - 1u ) );
+      const bool put = ( ( m >> w.lane ) & 1u ) && at < kGather;
+      if ( put )
+      {
+        sm.te[at] = te;
+        sm.tr[at] = r;
+        if constexpr ( STORED )
+        {
+#pragma unroll
+          for ( int a = 0; a < D; ++a ) copy_pair( &sm.e[at][2 * a], src + 2 * kLeafSize * a );
+        } else {
+          slabs_to_row< K, T, VT >( x.tverts, x.tV, te, x.eps, x.eps_hi, sm.e[at] );
+        }
+      }
+      w.ne = min( kGather, w.ne + __popc( m ) );
+      m &= ~__ballot_sync( 0xffffffffu, put );
+      if ( w.ne == kGather ) test_gathered( x, sm, w );
     }
   }
   __syncwarp();
 }
 
-// One packet in dense contact (see above). Returns false when the stack bound was reached (error raised).
-template< int K, typename T >
-__device__ __forceinline__ void traverse_packet_stored(const trav_args< T > &x, const uint32_t i0, const unsigned lane,
-                                                       dense_smem< K, T > &sm, const T *rb)
+// One packet: ranks i0 .. i0 + 31 against the target tree (see above). rb: the target root's slabs.
+template< int K, typename T, int VT, bool STORED >
+__device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint32_t i0, const unsigned lane,
+                                            walk_smem< K, T > &sm, const T *rb)
 {
   constexpr int D = K / 2;
-  constexpr int D0 = D < 4 ? D : 4;
-  constexpr int R16 = 2 * K * static_cast< int >( sizeof( T ) ) / 16;  // 16-byte pieces of a node row
   const uint32_t i = i0 + lane;
+  const T *wb = x.qwarp + static_cast< size_t >( i0 >> 5 ) * K;
+  // 1. The packet's union box against the target's root box (uniform over the warp).
   {
-    const T *wb = x.qwarp + static_cast< size_t >( i0 >> 5 ) * K;
     bool o = true;
 #pragma unroll
-    for ( int a = 0; a < D0; ++a ) o = o && ( __ldg( wb + 2 * a ) < rb[2 * a + 1] && rb[2 * a] < __ldg( wb + 2 * a + 1 ) );
-    if ( !o ) return;
-#pragma unroll
-    for ( int a = D0; a < D; ++a ) o = o && ( __ldg( wb + 2 * a ) < rb[2 * a + 1] && rb[2 * a] < __ldg( wb + 2 * a + 1 ) );
+    for ( int a = 0; a < D; ++a ) o = o && ( __ldg( wb + 2 * a ) < rb[2 * a + 1] && rb[2 * a] < __ldg( wb + 2 * a + 1 ) );
     if ( !o ) return;
   }
+  // 2. Each lane's own slabs (stored, or from its element's vertices) against the root box.
   const bool valid = i < x.nq;
-  T qlo[D], qhi[D];
-  bool in_root = valid;
+  const uint32_t qe = valid ? __ldg( x.qperm + i ) : 0u;
+  if constexpr ( STORED )
   {
-    const uint32_t iv = valid ? i : 0u;
+    const uint32_t iv = valid ? i : i0;
     const T *qs = x.qrows + static_cast< size_t >( iv >> 3 ) * ( kLeafSize * K ) + 2 * ( iv & 7u );
 #pragma unroll
-    for ( int a = 0; a < D; ++a )
-    {
-      load_pair( qs + 2 * kLeafSize * a, qlo[a], qhi[a] );
-      if ( !valid )
-      {
-        qlo[a] = T( 0 );
-        qhi[a] = T( 0 );
-      }
-      sm.q[lane][2 * a] = qlo[a];
-      sm.q[lane][2 * a + 1] = qhi[a];
-      in_root = in_root && ( qlo[a] < rb[2 * a + 1] && rb[2 * a] < qhi[a] );
-    }
-  }
-  sm.qe[lane] = valid ? __ldg( x.qperm + i ) : 0u;
-  const unsigned mask = __ballot_sync( 0xffffffffu, in_root );
-  if ( !mask ) return;
-  const int root = x.tsc->root;
-  int nleaf = 0;
-  uint32_t nout = 0;
-  if ( root < 0 )
-  {
-    if ( lane == 0 ) sm.leaf[0] = make_int2( ~root, static_cast< int >( mask ) );
-    flush_leaves< K, T >( x, sm, 1, i0, lane, nout );
-    drain_pairs< K, T >( x, sm, nout, lane );
-    return;
-  }
-  if ( lane == 0 ) sm.stack[0] = make_int2( root, static_cast< int >( mask ) );
-  int sp = 1;
-  while ( sp > 0 )
-  {
-    __syncwarp();
-    const int nb = sp < kDenseBatch< K, T > ? sp : kDenseBatch< K, T >;
-    sp -= nb;
-    // the batch's node rows into shared memory (one round of asynchronous copies), their links into registers
-    for ( int t = static_cast< int >( lane ); t < nb * R16; t += 32 )
-    {
-      const int k = t / R16, piece = t - k * R16;
-      const int node = sm.stack[sp + k].x;
-      cp_async16( reinterpret_cast< char * >( sm.rows[k] ) + 16 * piece,
-                  reinterpret_cast< const char * >( x.nbox + static_cast< size_t >( node ) * 2 * K ) + 16 * piece );
-    }
-    int2 links = make_int2( 0, 0 ), span = make_int2( 0, 0 );
-    if ( static_cast< int >( lane ) < nb )
-    {
-      const int node = sm.stack[sp + lane].x;
-      links = __ldg( x.child + node );
-      if ( x.self ) span = make_int2( node, __ldg( &x.range[node].y ) );
-    }
-    unsigned emask[kDenseBatch< K, T >];
-#pragma unroll
-    for ( int k = 0; k < kDenseBatch< K, T >; ++k ) emask[k] = k < nb ? static_cast< unsigned >( sm.stack[sp + k].y ) : 0u;
+    for ( int a = 0; a < D; ++a ) copy_pair( &sm.q[lane][2 * a], qs + 2 * kLeafSize * a );
     cp_async_wait_all();
+  } else {
+    if ( valid ) slabs_to_row< K, T, VT >( x.qverts, x.qV, qe, x.eps, x.eps_hi, sm.q[lane] );
+  }
+  sm.qe[lane] = qe;
+  if ( lane < K ) sm.g[lane] = __ldg( wb + lane );
+  __syncwarp();
+  bool in_root = valid;
+#pragma unroll
+  for ( int a = 0; a < D; ++a )
+  {
+    T ql, qh;
+    shared_pair( &sm.q[lane][2 * a], ql, qh );
+    in_root = in_root && ( ql < rb[2 * a + 1] && rb[2 * a] < qh );
+  }
+  walk_state w;
+  w.i0 = i0;
+  w.lane = lane;
+  w.in = __ballot_sync( 0xffffffffu, in_root );
+  if ( !w.in ) return;
+  const int root = x.tsc->root;
+  const unsigned lt = ( 1u << lane ) - 1u;
+  const int limit = STORED ? x.stack_limit : kWalkStack;
+  int sp = 0, nl = 0, nleaf = 0;
+  bool full = false;  // the stack bound was reached (uniform over the warp)
+  if ( lane == 0 )
+  {
+    if ( root < 0 ) sm.leaf[0] = ~root;
+    else sm.stack[0] = root;
+  }
+  if ( root < 0 ) nleaf = 1;
+  else sp = 1;
+  const T half = T( 0.5 ) * ( ( sm.g[1] - sm.g[0] ) + ( sm.g[3] - sm.g[2] ) + ( sm.g[5] - sm.g[4] ) );
+  while ( !full && ( sp > 0 || nl > 0 ) )
+  {
     __syncwarp();
-    unsigned m0[kDenseBatch< K, T >], m1[kDenseBatch< K, T >];
-#pragma unroll
-    for ( int k = 0; k < kDenseBatch< K, T >; ++k )
+    if ( nleaf > kLeafCap - 32 )
     {
-      if ( k >= nb ) break;
-      bool o0 = ( emask[k] >> lane ) & 1u, o1 = o0;
-      if ( x.self )
-      {
-        // left child covers buckets [l, node], right child [node + 1, r]: skip subtrees whose last rank <= i
-        const int node = __shfl_sync( 0xffffffffu, span.x, k ), last = __shfl_sync( 0xffffffffu, span.y, k );
-        o0 = o0 && kLeafSize * node + kLeafSize - 1 > static_cast< int >( i );
-        o1 = o1 && min( kLeafSize * last + kLeafSize - 1, static_cast< int >( x.nt ) - 1 ) > static_cast< int >( i );
-      }
-      // a chunk of slabs of the row is read from shared memory before it is tested
-      const T *row = sm.rows[k];
-#pragma unroll
-      for ( int a0 = 0; a0 < D; a0 += kNodeChunk< K, T > )
-      {
-        if ( !( o0 || o1 ) ) break;
-        T v[4 * kNodeChunk< K, T >];
-#pragma unroll
-        for ( int j = 0; j < kNodeChunk< K, T >; ++j )
-        {
-          if ( a0 + j >= D ) break;
-          shared_pair( row + 4 * ( a0 + j ), v[4 * j], v[4 * j + 1] );
-          shared_pair( row + 4 * ( a0 + j ) + 2, v[4 * j + 2], v[4 * j + 3] );
-        }
-#pragma unroll
-        for ( int j = 0; j < kNodeChunk< K, T >; ++j )
-        {
-          if ( a0 + j >= D ) break;
-          o0 = o0 && ( qlo[a0 + j] < v[4 * j + 1] && v[4 * j] < qhi[a0 + j] );
-          o1 = o1 && ( qlo[a0 + j] < v[4 * j + 3] && v[4 * j + 2] < qhi[a0 + j] );
-        }
-      }
-      m0[k] = __ballot_sync( 0xffffffffu, o0 );
-      m1[k] = __ballot_sync( 0xffffffffu, o1 );
-    }
-    // children: buckets to the leaf queue, internal nodes onto the stack (warp-uniform; lane 0 writes)
-#pragma unroll
-    for ( int k = 0; k < kDenseBatch< K, T >; ++k )
-    {
-      if ( k >= nb ) break;
-      const int cx = __shfl_sync( 0xffffffffu, links.x, k ), cy = __shfl_sync( 0xffffffffu, links.y, k );
-#pragma unroll
-      for ( int side = 0; side < 2; ++side )
-      {
-        const unsigned m = side ? m1[k] : m0[k];
-        const int ch = side ? cy : cx;
-        if ( !m ) continue;
-        if ( ch < 0 )
-        {
-          if ( lane == 0 ) sm.leaf[nleaf] = make_int2( ~ch, static_cast< int >( m ) );
-          ++nleaf;
-        } else {
-          if ( sp >= x.dense_stack )
-          {
-            if ( lane == 0 ) atomicCAS( &x.ps->error, 0, kErrOverflowStack );
-            drain_pairs< K, T >( x, sm, nout, lane );
-            return;
-          }
-          if ( lane == 0 ) sm.stack[sp] = make_int2( ch, static_cast< int >( m ) );
-          ++sp;
-        }
-      }
-    }
-    if ( nleaf > kLeafQueue - 2 * kDenseBatch< K, T > )
-    {
-      flush_leaves< K, T >( x, sm, nleaf, i0, lane, nout );
+      filter_buckets< K, T, VT, STORED >( x, sm, w, nleaf );
       nleaf = 0;
     }
+    const bool wide = sp + nl + 32 + kWalkDepth <= limit;
+    if ( sp > 0 && nl <= kCheckCap - 32 && ( wide || nl == 0 ) )
+    {
+      // expand: lane = (node, child), the child against the packet's union box
+      const int p = wide ? min( sp, 16 ) : 1;
+      const int k = static_cast< int >( lane >> 1 ), side = static_cast< int >( lane & 1u );
+      bool o = k < p;
+      const int node = o ? sm.stack[sp - 1 - k] : 0;
+      sp -= p;
+      int c = 0;
+      bool small = false;
+      if ( o )
+      {
+        c = __ldg( reinterpret_cast< const int * >( x.child ) + 2 * node + side );
+        const T *nb = x.nbox + static_cast< size_t >( node ) * D * 4 + 2 * side;
+        T lo[D], hi[D];
+#pragma unroll
+        for ( int a = 0; a < D; ++a ) load_pair( nb + a * 4, lo[a], hi[a] );
+        if ( x.self )
+        {
+          // left child covers buckets [l, node], right child [node + 1, r]: skip subtrees whose last rank <= i0
+          const int last = side ? __ldg( &x.range[node].y ) : node;
+          o = min( kLeafSize * last + kLeafSize - 1, static_cast< int >( x.nt ) - 1 ) > static_cast< int >( i0 );
+        }
+        small = ( hi[0] - lo[0] ) + ( hi[1] - lo[1] ) + ( hi[2] - lo[2] ) < half;
+        bool lo_ok = true, hi_ok = true;  // bitwise: no branch per comparison
+#pragma unroll
+        for ( int a = 0; a < D; ++a )
+        {
+          T gl, gh;
+          shared_pair( &sm.g[2 * a], gl, gh );
+          lo_ok &= gl < hi[a];
+          hi_ok &= lo[a] < gh;
+        }
+        o = o & lo_ok & hi_ok;
+      }
+      const unsigned ml = __ballot_sync( 0xffffffffu, o && small );
+      const unsigned mp = __ballot_sync( 0xffffffffu, o && !small && c >= 0 );
+      const unsigned mb = __ballot_sync( 0xffffffffu, o && !small && c < 0 );
+      full = sp + __popc( mp ) > limit;
+      if ( full ) break;
+      if ( o )
+      {
+        if ( small ) sm.list[nl + __popc( ml & lt )] = make_int2( 2 * node + side, c );
+        else if ( c >= 0 ) sm.stack[sp + __popc( mp & lt )] = c;
+        else sm.leaf[nleaf + __popc( mb & lt )] = ~c;
+      }
+      nl += __popc( ml );
+      sp += __popc( mp );
+      nleaf += __popc( mb );
+      continue;
+    }
+    // check: lane = query, the listed boxes' cardinal slabs against every query of the packet
+    for ( int b0 = 0; b0 < nl && !full; b0 += kCheckRows )
+    {
+      const int nb = min( kCheckRows, nl - b0 );
+      {
+        static_assert( kCheckRows * 3 <= 32, "one pair per lane" );
+        const int k = static_cast< int >( lane ) / 3, a = static_cast< int >( lane ) - 3 * k;
+        if ( k < nb )
+        {
+          const int e = sm.list[b0 + k].x;
+          copy_pair( &sm.rows[k][2 * a], x.nbox + static_cast< size_t >( e >> 1 ) * D * 4 + a * 4 + ( e & 1 ) * 2 );
+        }
+      }
+      cp_async_wait_all();
+      __syncwarp();
+      unsigned alive = in_root ? ( 1u << nb ) - 1u : 0u;
+#pragma unroll
+      for ( int a = 0; a < 3; ++a )
+      {
+        T ql, qh;
+        shared_pair( &sm.q[lane][2 * a], ql, qh );
+#pragma unroll
+        for ( int j = 0; j < kCheckRows; ++j )
+        {
+          T bl, bh;
+          shared_pair( &sm.rows[j][2 * a], bl, bh );
+          const bool o = ( ql < bh ) & ( bl < qh );
+          alive &= o ? ~0u : ~( 1u << j );
+        }
+      }
+      alive = __reduce_or_sync( 0xffffffffu, alive );  // bit j: some query overlaps box j
+      for ( int j = 0; j < nb; ++j )
+      {
+        if ( !( ( alive >> j ) & 1u ) ) continue;
+        const int ch = sm.list[b0 + j].y;
+        if ( ch < 0 )
+        {
+          if ( nleaf == kLeafCap )
+          {
+            __syncwarp();
+            filter_buckets< K, T, VT, STORED >( x, sm, w, nleaf );
+            nleaf = 0;
+          }
+          if ( lane == 0 ) sm.leaf[nleaf] = ~ch;
+          ++nleaf;
+        } else if ( sp < limit ) {
+          if ( lane == 0 ) sm.stack[sp] = ch;
+          ++sp;
+        } else {
+          full = true;
+        }
+      }
+      __syncwarp();  // the rows are refilled by the next boxes
+    }
+    nl = 0;
   }
-  if ( nleaf > 0 ) flush_leaves< K, T >( x, sm, nleaf, i0, lane, nout );
-  drain_pairs< K, T >( x, sm, nout, lane );
+  __syncwarp();
+  filter_buckets< K, T, VT, STORED >( x, sm, w, nleaf );
+  if ( w.ne ) test_gathered( x, sm, w );
+  if ( full && lane == 0 ) atomicCAS( &x.ps->error, 0, kErrOverflowStack );
+  drain_pairs( x, sm, w );
 }
 
-// Resident blocks per SM of the dense walk: as many as its shared memory allows (228 KB per SM, 1 KB of it reserved
-// per block), at most kDenseBlockCap; the register budget follows from it. 18-DOP FP64 rows run at 5 blocks (96
-// registers, no spills): at 6 they were squeezed into 80 registers with spills, and the walk was 16% slower.
+// Roots first: objects far apart (most pairs of a batch) end here for the whole grid. No tree exists after a failed
+// sort of either object.
 template< int K, typename T >
-constexpr int kDenseBlockCap = ( K == 18 && sizeof( T ) == 8 ) ? 5 : 6;
-template< int K, typename T >
-constexpr int kDenseBlocksBySmem =
-  ( 228 * 1024 ) / ( ( kTravThreads / 32 ) * static_cast< int >( sizeof( dense_smem< K, T > ) ) + 1024 );
-template< int K, typename T >
-constexpr int kDenseBlocksPerSM =
-  kDenseBlocksBySmem< K, T > < kDenseBlockCap< K, T > ? kDenseBlocksBySmem< K, T > : kDenseBlockCap< K, T >;
+__device__ __forceinline__ bool objects_meet(const trav_args< T > &x, const obj_scalars *__restrict__ qsc)
+{
+  if ( *reinterpret_cast< const volatile int * >( &x.tsc->error ) == kErrTimeout ||
+       *reinterpret_cast< const volatile int * >( &qsc->error ) == kErrTimeout )
+    return false;
+  constexpr int D0 = K / 2 < 4 ? K / 2 : 4;
+  const T *rb = reinterpret_cast< const T * >( x.tsc->root_box );
+  const T *qr = reinterpret_cast< const T * >( qsc->root_box );
+  bool o = true;
+#pragma unroll
+  for ( int a = 0; a < D0; ++a ) o = o && ( qr[2 * a] < rb[2 * a + 1] && rb[2 * a] < qr[2 * a + 1] );
+  return o;
+}
 
-// Dense contact: one warp per packet of 32 query ranks (the hardware balances the walks).
+// Sparse contact: a persistent grid. A warp takes chunks from the pair counters' packet dispenser; chunk c holds the
+// packets c, c + C, c + 2C, ... (C chunks), so a contact region (consecutive Morton ranks) is spread over many chunks.
+// Lane j tests the union box of the chunk's packet j against the target root (one load per lane for the packets far
+// from the target), then the warp walks the survivors one after the other.
+template< int K, typename T, int VT >
+__device__ void traverse_body(const trav_item &item, uint32_t, uint32_t)
+{
+  const trav_args< T > x = typed< T >( item );
+  constexpr int D = K / 2;
+  extern __shared__ __align__( 16 ) unsigned char s_walk[];
+  auto &sm = reinterpret_cast< walk_smem< K, T > * >( s_walk )[threadIdx.x >> 5];
+  const unsigned lane = threadIdx.x & 31u;
+  if ( !objects_meet< K, T >( x, item.qsc ) ) return;
+  const T *rb = reinterpret_cast< const T * >( x.tsc->root_box );
+  const uint32_t packets = ( x.nq + 31 ) / 32;
+  const uint32_t chunks = ( packets + 31 ) / 32;
+  while ( true )
+  {
+    uint32_t c = 0;
+    if ( lane == 0 ) c = atomicAdd( &x.ps->packet_next, 1u );
+    c = __shfl_sync( 0xffffffffu, c, 0 );
+    if ( c >= chunks ) break;
+    const uint64_t pk = c + static_cast< uint64_t >( lane ) * chunks;
+    bool o = false;
+    if ( pk < packets )
+    {
+      const T *wb = x.qwarp + pk * D * 2;
+      o = true;
+#pragma unroll
+      for ( int a = 0; a < D; ++a ) o = o && ( __ldg( wb + 2 * a ) < rb[2 * a + 1] && rb[2 * a] < __ldg( wb + 2 * a + 1 ) );
+    }
+    for ( unsigned m = __ballot_sync( 0xffffffffu, o ); m; m &= m - 1 )
+    {
+      const uint32_t p = c + static_cast< uint32_t >( __ffs( m ) - 1 ) * chunks;
+      walk_packet< K, T, VT, false >( x, p * 32, lane, sm, rb );
+    }
+  }
+}
+
+// Dense contact: one warp per packet (the hardware balances the walks).
 template< int K, typename T >
 __device__ void stored_body(const trav_item &item, uint32_t bid, uint32_t)
 {
   const trav_args< T > x = typed< T >( item );
-  const obj_scalars *__restrict__ qsc = item.qsc;
-  constexpr int D = K / 2;
-  constexpr int D0 = D < 4 ? D : 4;
-  constexpr int WPB = kTravThreads / 32;
-  __shared__ __align__( 16 ) dense_smem< K, T > s_dense[WPB];
+  extern __shared__ __align__( 16 ) unsigned char s_walk[];
+  auto &sm = reinterpret_cast< walk_smem< K, T > * >( s_walk )[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31u;
-  if ( *reinterpret_cast< const volatile int * >( &x.tsc->error ) == kErrTimeout ||
-       *reinterpret_cast< const volatile int * >( &qsc->error ) == kErrTimeout )
-    return;
+  if ( !objects_meet< K, T >( x, item.qsc ) ) return;
   const T *rb = reinterpret_cast< const T * >( x.tsc->root_box );
-  {
-    const T *qr = reinterpret_cast< const T * >( qsc->root_box );
-    bool o = true;
-#pragma unroll
-    for ( int a = 0; a < D0; ++a ) o = o && ( qr[2 * a] < rb[2 * a + 1] && rb[2 * a] < qr[2 * a + 1] );
-    if ( !o ) return;
-  }
   const uint32_t packets = ( x.nq + 31 ) / 32;
   const uint32_t pk = ( bid * blockDim.x + threadIdx.x ) >> 5;
-  if ( pk < packets ) traverse_packet_stored< K, T >( x, pk * 32, lane, s_dense[threadIdx.x >> 5], rb );
+  if ( pk < packets ) walk_packet< K, T, 0, true >( x, pk * 32, lane, sm, rb );
 }
+
+// Shared memory per block of the walks, and their resident blocks per SM: as many as it allows (228 KB per SM, 1 KB of
+// it reserved per block) up to a cap that keeps the registers without spills.
+template< int K, typename T, bool STORED >
+constexpr int kWalkSmem = ( kTravThreads / 32 ) * static_cast< int >( sizeof( walk_smem< K, T > ) );
+template< int K, typename T, bool STORED >
+constexpr int kWalkBySmem = ( 228 * 1024 ) / ( kWalkSmem< K, T, STORED > + 1024 );
+template< int K, typename T, bool STORED >
+constexpr int kWalkCap = STORED ? ( sizeof( T ) == 4 ? 8 : 6 ) * 128 / kTravThreads : kTravBlocksPerSM;
+template< int K, typename T, bool STORED >
+constexpr int kWalkBlocks = kWalkBySmem< K, T, STORED > < kWalkCap< K, T, STORED > ? kWalkBySmem< K, T, STORED >
+                                                                                  : kWalkCap< K, T, STORED >;
 
 // One scene's item and grid. Dense contact: one warp per packet. Sparse: a persistent grid of at most the resident
 // blocks (4 per SM), one warp per chunk of 32 packets at most.
@@ -806,7 +710,7 @@ void trav_item_t(tree_view q, tree_view t, bool self, bool dense, double eps, ui
   it->pairs = pairs;
   it->cap = cap;
   it->ps = ps;
-  it->dense_stack = dense_stack_limit > 0 && dense_stack_limit < kDenseStack ? dense_stack_limit : kDenseStack;
+  it->dense_stack = dense_stack_limit > 0 && dense_stack_limit < kWalkStack ? dense_stack_limit : kWalkStack;
   it->qsc = q.sc;
   constexpr uint64_t kWarps = kTravThreads / 32;
   const uint64_t packets = ( q.n + 31 ) / 32;
@@ -819,6 +723,52 @@ void trav_item_t(tree_view q, tree_view t, bool self, bool dense, double eps, ui
   *dense_out = dense;
 }
 
+// The shared-memory opt-in of a walk's two launch forms, once per device.
+template< int K, typename T, int VT, bool STORED >
+struct walk_kernels
+{
+  static constexpr int MB = kWalkBlocks< K, T, STORED >;
+  static constexpr int smem = kWalkSmem< K, T, STORED >;
+  static constexpr auto single()
+  {
+    if constexpr ( STORED ) return &k_single< trav_item, stored_body< K, T >, kTravThreads, MB >;
+    else return &k_single< trav_item, traverse_body< K, T, VT >, kTravThreads, MB >;
+  }
+  static constexpr auto batched()
+  {
+    if constexpr ( STORED ) return &k_batched< trav_item, stored_body< K, T >, kTravThreads, MB >;
+    else return &k_batched< trav_item, traverse_body< K, T, VT >, kTravThreads, MB >;
+  }
+  static cudaError_t setup()
+  {
+    if constexpr ( smem <= 47 * 1024 ) return cudaSuccess;
+    static std::atomic< unsigned long long > configured{ 0 };
+    int dev = 0;
+    cudaError_t e = cudaGetDevice( &dev );
+    if ( e != cudaSuccess ) return e;
+    const unsigned long long bit = 1ull << ( dev & 63 );
+    if ( configured.load() & bit ) return cudaSuccess;
+    e = cudaFuncSetAttribute( single(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
+    if ( e == cudaSuccess ) e = cudaFuncSetAttribute( batched(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
+    if ( e == cudaSuccess ) configured.fetch_or( bit );
+    return e;
+  }
+  static cudaError_t launch(const trav_item &it, uint32_t grid, cudaStream_t s)
+  {
+    const cudaError_t e = setup();
+    if ( e != cudaSuccess ) return e;
+    single()<<< grid, kTravThreads, smem, s >>>( it );
+    return cudaGetLastError();
+  }
+  static cudaError_t launch_batch(const batch_launch &b, cudaStream_t s)
+  {
+    const cudaError_t e = setup();
+    if ( e != cudaSuccess ) return e;
+    batched()<<< b.blocks, kTravThreads, smem, s >>>( static_cast< const trav_item * >( b.items ), b.starts, b.nitems );
+    return cudaGetLastError();
+  }
+};
+
 template< int K, typename T >
 cudaError_t launch_trav_t(tree_view q, tree_view t, bool self, bool dense, double eps, uint2 *pairs, uint64_t cap,
                           pair_scalars *ps, cudaStream_t s, int dense_stack_limit)
@@ -826,42 +776,29 @@ cudaError_t launch_trav_t(tree_view q, tree_view t, bool self, bool dense, doubl
   trav_item it;
   uint32_t grid = 0;
   trav_item_t< K, T >( q, t, self, dense, eps, pairs, cap, ps, dense_stack_limit, &it, &grid, &dense );
-  // both objects' element slabs stored (dense contact): the batched walk that only reads them; else the one that
-  // computes the slabs it tests from the vertices (unrolled when both objects have the same vertex count)
-  if ( dense )
+  // both objects' element slabs stored (dense contact): the walk that only reads them; else the one that computes the
+  // slabs it tests from the vertices (unrolled when both objects have the same vertex count)
+  if ( dense ) return walk_kernels< K, T, 0, true >::launch( it, grid, s );
+  switch ( q.V == t.V ? q.V : 0 )
   {
-    k_single< trav_item, stored_body< K, T >, kTravThreads, kDenseBlocksPerSM< K, T > ><<< grid, kTravThreads, 0, s >>>( it );
-    return cudaGetLastError();
+    case 3: return walk_kernels< K, T, 3, false >::launch( it, grid, s );
+    case 4: return walk_kernels< K, T, 4, false >::launch( it, grid, s );
+    case 8: return walk_kernels< K, T, 8, false >::launch( it, grid, s );
+    default: return walk_kernels< K, T, 0, false >::launch( it, grid, s );
   }
-  const uint32_t V = q.V == t.V ? q.V : 0;
-  switch ( V )
-  {
-    case 3: k_single< trav_item, traverse_body< K, T, 3 >, kTravThreads, kTravBlocksPerSM ><<< grid, kTravThreads, 0, s >>>( it ); break;
-    case 4: k_single< trav_item, traverse_body< K, T, 4 >, kTravThreads, kTravBlocksPerSM ><<< grid, kTravThreads, 0, s >>>( it ); break;
-    case 8: k_single< trav_item, traverse_body< K, T, 8 >, kTravThreads, kTravBlocksPerSM ><<< grid, kTravThreads, 0, s >>>( it ); break;
-    default: k_single< trav_item, traverse_body< K, T, 0 >, kTravThreads, kTravBlocksPerSM ><<< grid, kTravThreads, 0, s >>>( it ); break;
-  }
-  return cudaGetLastError();
 }
 
 template< int K, typename T >
 cudaError_t launch_trav_batch_t(bool dense, uint32_t V, const batch_launch &b, cudaStream_t s)
 {
-  const trav_item *items = static_cast< const trav_item * >( b.items );
-  if ( dense )
-  {
-    k_batched< trav_item, stored_body< K, T >, kTravThreads, kDenseBlocksPerSM< K, T > ><<< b.blocks, kTravThreads, 0, s >>>(
-      items, b.starts, b.nitems );
-    return cudaGetLastError();
-  }
+  if ( dense ) return walk_kernels< K, T, 0, true >::launch_batch( b, s );
   switch ( V )
   {
-    case 3: k_batched< trav_item, traverse_body< K, T, 3 >, kTravThreads, kTravBlocksPerSM ><<< b.blocks, kTravThreads, 0, s >>>( items, b.starts, b.nitems ); break;
-    case 4: k_batched< trav_item, traverse_body< K, T, 4 >, kTravThreads, kTravBlocksPerSM ><<< b.blocks, kTravThreads, 0, s >>>( items, b.starts, b.nitems ); break;
-    case 8: k_batched< trav_item, traverse_body< K, T, 8 >, kTravThreads, kTravBlocksPerSM ><<< b.blocks, kTravThreads, 0, s >>>( items, b.starts, b.nitems ); break;
-    default: k_batched< trav_item, traverse_body< K, T, 0 >, kTravThreads, kTravBlocksPerSM ><<< b.blocks, kTravThreads, 0, s >>>( items, b.starts, b.nitems ); break;
+    case 3: return walk_kernels< K, T, 3, false >::launch_batch( b, s );
+    case 4: return walk_kernels< K, T, 4, false >::launch_batch( b, s );
+    case 8: return walk_kernels< K, T, 8, false >::launch_batch( b, s );
+    default: return walk_kernels< K, T, 0, false >::launch_batch( b, s );
   }
-  return cudaGetLastError();
 }
 
 // The vertices of one element into registers: 16-byte loads when every element starts on a 16-byte boundary (an
