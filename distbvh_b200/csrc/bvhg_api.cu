@@ -952,7 +952,7 @@ bvhg_status capture_batch_fused(bvhg_ctx *ctx, batch_state &B, const batch_args 
     }
     fg.slabs.push_back( slabs_args{ o.verts, o.V, n, eps, f32_round_up( eps ), o.sorted_vals(), o.bucket_box.p,
                                     o.warp_box.p, o.store_slabs ? o.elem_cache.p : nullptr, o.sc() } );
-    fg.b_slabs.push_back( slabs_blocks( n ) );
+    fg.b_slabs.push_back( slabs_blocks( K, fp32, V, n ) );
     o.stored = o.store_slabs;
     if ( m > 1 )
     {

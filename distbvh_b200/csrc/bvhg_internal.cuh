@@ -332,7 +332,7 @@ cudaError_t launch_climb(int K, bool fp32, uint64_t n, const uint8_t *bdel, void
 
 // Batched forms of the slab kernel (items: slabs_args; one V for all items), the block-local build, the climb and
 // the refit (items: tree_args of objects with more than one bucket), with the blocks of one item.
-uint32_t slabs_blocks(uint64_t n);
+uint32_t slabs_blocks(int K, bool fp32, uint32_t V, uint64_t n);
 cudaError_t launch_slabs_batch(int K, bool fp32, uint32_t V, const batch_launch &b, cudaStream_t s);
 uint32_t build_blocks(uint64_t n);
 cudaError_t launch_build_batch(int K, bool fp32, const batch_launch &b, cudaStream_t s);

@@ -18,8 +18,10 @@
 #include "bulk_copy.cuh"
 #include "kdop_math.cuh"
 
-namespace bvhg {
+#include <atomic>
 
+namespace bvhg {
+int device_sm_count();
 namespace {
 
 constexpr int kBuildThreads = 128;
@@ -139,20 +141,122 @@ __device__ __forceinline__ long long cdelta(const uint8_t *__restrict__ bdel, in
   return ( static_cast< long long >( __ldg( bdel + b ) ) << 32 ) | static_cast< unsigned >( b );
 }
 
-constexpr int kSlabThreads = 128;  // ranks per block of the element slab kernel
+constexpr int kSlabThreads = 128;  // threads per block of the element slab kernel
+constexpr int kSlabWarps = kSlabThreads / 32;
 
-// Element slabs in rank order, one thread per rank (the element perm[r] of rank r), staged in shared memory (padded
-// to C + 1 components against bank conflicts); per block of 128 ranks, the unions of its 16 leaf buckets and its 4
-// query groups of 32 ranks are written out coalesced: bucket_box row b and warp_box row g each hold the C = 2 D
-// values (min, max) per slab. The element slabs themselves go to elem_rows (slab-major per leaf bucket: rank
-// r = 8 b + j, slab a at elem_rows[b * 8 C + 16 a + 2 j + {0 min, 1 max}]) only when given (objects in dense
-// contact, whose traversals test most buckets); otherwise the traversal computes the few it tests from the
-// vertices. A one-bucket object also gets its root box here. A rank whose index is not an element index marks a failed sort.
-template< int K, int VT >
-constexpr int kSlabMinBlocks = ( VT == 3 && K <= 18 ) ? 8 : ( VT == 8 ? 3 : 4 );
+// Shared-memory stride of one element's staged vertices, in doubles: elements of 4 and 8 vertices are padded by 16
+// bytes, so that the 16-byte reads of 8 neighbouring threads fall into different banks (an odd stride of 9 doubles
+// needs no padding).
+template< int VT >
+constexpr int kVertStride = VT == 0 ? 0 : ( VT % 2 == 0 ? VT * 3 + 2 : VT * 3 );
 
+// Shared memory of one warp of the slab kernel: its staged vertices and its 32 element rows (K values each: rows of 9
+// and 13 pairs need no padding, the pairs of 8 neighbouring rows fall into different banks).
 template< int K, typename T, int VT >
-__device__ void slabs_body(const slabs_args &args, uint32_t bid, uint32_t)
+constexpr int kSlabWarpVerts = 32 * kVertStride< VT > * 8;
+template< int K, typename T, int VT >
+constexpr int kSlabWarpSmem = kSlabWarpVerts< K, T, VT > + 32 * K * static_cast< int >( sizeof( T ) );
+template< int K, typename T, int VT >
+constexpr int kSlabSmem = kSlabWarps * kSlabWarpSmem< K, T, VT >;
+
+// Resident blocks per SM: what shared memory allows (1 KB of it reserved per block), at most 8 (64 registers).
+template< int K, typename T, int VT >
+constexpr int kSlabBySmem = ( 228 * 1024 ) / ( kSlabSmem< K, T, VT > + 1024 );
+template< int K, typename T, int VT >
+constexpr int kSlabCap = VT == 0 ? 4 : ( VT == 8 ? 5 : 8 );
+template< int K, typename T, int VT >
+constexpr int kSlabBlocks = kSlabBySmem< K, T, VT > < kSlabCap< K, T, VT > ? kSlabBySmem< K, T, VT > : kSlabCap< K, T, VT >;
+
+// LANES neighbouring lanes copy LANES neighbouring pieces (BYTES each, from piece FIRST on) of one of the 32 elements
+// e (one per lane, the first `rows` of them): 32 / LANES elements per instruction, whose place needs no division.
+template< int VT, int BYTES, int FIRST, int LANES >
+__device__ __forceinline__ void gather_pieces(const double *__restrict__ verts, uint32_t e, int rows, double *s_v, int lane)
+{
+  constexpr int PER = 32 / LANES;
+  const int w = ( FIRST + ( lane & ( LANES - 1 ) ) ) * ( BYTES / 8 ), q0 = lane / LANES;
+#pragma unroll
+  for ( int i = 0; i < LANES; ++i )
+  {
+    const int q = PER * i + q0;
+    const uint32_t eq = __shfl_sync( 0xffffffffu, e, q );
+    const double *src = verts + static_cast< size_t >( eq ) * ( VT * 3 ) + w;
+    if ( q < rows )
+    {
+      if constexpr ( BYTES == 16 ) cp_async16( s_v + q * kVertStride< VT > + w, src );
+      else cp_async_small< 8 >( s_v + q * kVertStride< VT > + w, src );
+    }
+  }
+}
+
+// The vertices of the 32 elements e into s_v by asynchronous copies.
+template< int VT >
+__device__ __forceinline__ void gather_vertices(const double *__restrict__ verts, uint32_t e, int rows, double *s_v, int lane)
+{
+  if constexpr ( VT % 2 == 0 )
+  {
+    // 6 or 12 pieces of 16 bytes
+    if ( ( reinterpret_cast< uintptr_t >( verts ) & 15 ) == 0 )
+    {
+      if constexpr ( VT == 4 )
+      {
+        gather_pieces< VT, 16, 0, 4 >( verts, e, rows, s_v, lane );
+        gather_pieces< VT, 16, 4, 2 >( verts, e, rows, s_v, lane );
+      } else {
+        gather_pieces< VT, 16, 0, 8 >( verts, e, rows, s_v, lane );
+        gather_pieces< VT, 16, 8, 4 >( verts, e, rows, s_v, lane );
+      }
+      return;
+    }
+  }
+  // 9, 12 or 24 pieces of 8 bytes
+  gather_pieces< VT, 8, 0, 8 >( verts, e, rows, s_v, lane );
+  if constexpr ( VT == 3 ) gather_pieces< VT, 8, 8, 1 >( verts, e, rows, s_v, lane );
+  else if constexpr ( VT == 4 ) gather_pieces< VT, 8, 8, 4 >( verts, e, rows, s_v, lane );
+  else
+  {
+    gather_pieces< VT, 8, 8, 8 >( verts, e, rows, s_v, lane );
+    gather_pieces< VT, 8, 16, 8 >( verts, e, rows, s_v, lane );
+  }
+}
+
+// This lane's staged vertices into registers.
+template< int VT >
+__device__ __forceinline__ void staged_vertices(const double *s_v, int q, double *v)
+{
+  const double *src = s_v + q * kVertStride< VT >;
+  if constexpr ( VT % 2 == 0 )
+  {
+#pragma unroll
+    for ( int k = 0; k < VT * 3; k += 2 )
+    {
+      const double2 t = *reinterpret_cast< const double2 * >( src + k );
+      v[k] = t.x;
+      v[k + 1] = t.y;
+    }
+  } else {
+#pragma unroll
+    for ( int k = 0; k < VT * 3; ++k ) v[k] = src[k];
+  }
+}
+
+// Element slabs in rank order: a warp takes groups of 32 ranks (one lane per rank, the element perm[r] of rank r), and
+// writes the unions of the group's 4 leaf buckets and of the whole group (bucket_box row b and warp_box row g each
+// hold the C = 2 D values (min, max) per slab). The element slabs themselves go to elem_rows only when given (objects
+// in dense contact, whose traversals test most buckets; layout below); otherwise the traversal computes the few it
+// tests from the vertices. A one-bucket object also gets its root box here. A rank whose index is not an element index
+// marks a failed sort.
+//
+// What bounds it is the gather and the traffic through shared memory. The grid is persistent and a warp keeps a gather
+// in flight while it works: the indices of its next group are loaded a group ahead, and the next group's vertices
+// start to stream into shared memory as soon as this group's are in registers. Nothing synchronises the warps of a
+// block, and rows are written and united as (min, max) pairs. The FP64 slabs share their products and skip the
+// products by 0 and 1 (vertex_slabs): the same values with less than half the operations. Both objects of 8.4M
+// tetrahedra, 26-DOP FP64 with stored rows: 1.64 -> 1.33 ms; 2.1M each, 18-DOP FP32: 0.215 -> 0.170 ms; 200,003
+// tetrahedra 23 -> 19 us; 9.4M triangles, 18-DOP FP64: 0.309 -> 0.303 ms (67% of the shared-memory wavefronts). One
+// thread loading its element 8 bytes at a time was the previous gather; the same copies without the overlap took
+// 0.339 ms for the triangles.
+template< int K, typename T, int VT >
+__device__ void slabs_body(const slabs_args &args, uint32_t bid, uint32_t nblk)
 {
   const double *__restrict__ verts = args.verts;
   const uint32_t Vrt = args.V;
@@ -160,99 +264,132 @@ __device__ void slabs_body(const slabs_args &args, uint32_t bid, uint32_t)
   const double eps = args.eps;
   const float eps_hi = args.eps_hi;
   const uint32_t *__restrict__ vals = args.vals;
-  T *__restrict__ bucket_box = static_cast< T * >( args.bucket_box );
-  T *__restrict__ warp_box = static_cast< T * >( args.warp_box );
   T *__restrict__ elem_rows = static_cast< T * >( args.elem_rows );
   obj_scalars *sc = args.sc;
   constexpr int D = K / 2;
   constexpr int C = 2 * D;
-  constexpr int P = C + 1;
   constexpr int G = 32 / kLeafSize;  // buckets per query group
   using io = box_io< T >;
-  __shared__ T s_el[kSlabThreads * P];
-  __shared__ T s_bk[( kSlabThreads / kLeafSize ) * P];
+  extern __shared__ __align__( 16 ) unsigned char s_slab[];
   if ( *reinterpret_cast< volatile int * >( &sc->error ) == kErrTimeout ) return;  // no valid permutation
-  const int tid = threadIdx.x;
-  const int r0 = static_cast< int >( bid ) * kSlabThreads;
-  const int rows = min( kSlabThreads, n - r0 );
-  if ( tid < rows )
-  {
-    const uint32_t e = __ldg( vals + r0 + tid );
-    T lo[D], hi[D];
-    if ( e < static_cast< uint32_t >( n ) )
+  const int lane = static_cast< int >( threadIdx.x & 31u ), warp = static_cast< int >( threadIdx.x >> 5 );
+  double *s_v = reinterpret_cast< double * >( s_slab + warp * kSlabWarpSmem< K, T, VT > );
+  T *s_el = reinterpret_cast< T * >( s_slab + warp * kSlabWarpSmem< K, T, VT > + kSlabWarpVerts< K, T, VT > );
+  const int groups = ( n + 31 ) / 32, stride = static_cast< int >( nblk ) * kSlabWarps;
+  int g = static_cast< int >( bid ) * kSlabWarps + warp;
+  if ( g >= groups ) return;
+  bool bad = false;
+  auto element = [&](int group) -> uint32_t {
+    const int r = 32 * group + lane;
+    uint32_t e = group < groups && r < n ? __ldg( vals + r ) : 0u;
+    if ( e >= static_cast< uint32_t >( n ) )
     {
-      leaf_slabs< K, T, VT >( verts, Vrt, e, eps, eps_hi, lo, hi );
+      bad = true;
+      e = 0u;
+    }
+    return e;
+  };
+  uint32_t e = element( g ), en = element( g + stride );
+  if constexpr ( VT > 0 ) gather_vertices< VT >( verts, e, min( 32, n - 32 * g ), s_v, lane );
+  for ( ; g < groups; g += stride )
+  {
+    const int r0 = 32 * g;
+    const int rows = min( 32, n - r0 );
+    T *row = s_el + lane * C;
+    if constexpr ( VT > 0 )
+    {
+      double v[VT * 3];
+      cp_async_wait_all();
+      __syncwarp();
+      staged_vertices< VT >( s_v, lane < rows ? lane : 0, v );
+      __syncwarp();
+      if ( g + stride < groups ) gather_vertices< VT >( verts, en, min( 32, n - 32 * ( g + stride ) ), s_v, lane );
+      vertex_slabs< K, T, VT >( v, eps, eps_hi, row );
     } else {
-      atomicCAS( &sc->error, 0, kErrTimeout );
-      const T inf = static_cast< T >( __longlong_as_double( 0x7ff0000000000000LL ) );
+      T lo[D], hi[D];
+      leaf_slabs< K, T, VT >( verts, Vrt, e, eps, eps_hi, lo, hi );
 #pragma unroll
-      for ( int a = 0; a < D; ++a )
+      for ( int a = 0; a < D; ++a ) io::store2( row + 2 * a, lo[a], hi[a] );
+    }
+    e = en;
+    en = element( g + 2 * stride );
+    __syncwarp();
+    const int nb = ( rows + kLeafSize - 1 ) / kLeafSize;
+    if ( elem_rows )
+    {
+      // slab-major per leaf bucket ([bucket][slab][element j < 8][min, max]): the walk over stored slabs reads one slab
+      // of eight elements as one piece
+      T *er = elem_rows + static_cast< size_t >( r0 ) * C;
+      for ( int k = lane; k < nb * kLeafSize * D; k += 32 )
       {
-        lo[a] = inf;
-        hi[a] = -inf;
+        const int lb = k / ( kLeafSize * D ), rem = k - lb * ( kLeafSize * D );
+        const int a = rem / kLeafSize, q = lb * kLeafSize + ( rem & ( kLeafSize - 1 ) );
+        if ( q < rows )
+        {
+          T lo, hi;
+          io::load2( s_el + q * C + 2 * a, lo, hi );
+          io::store2( er + 2 * k, lo, hi );
+        }
+      }
+      __syncwarp();  // the unions below overwrite each bucket's first row
+    }
+    // bucket unions (ranks in order, as the serial union of the reference merges them), one (min, max) pair per lane,
+    // left in the bucket's first row
+    T *bb = static_cast< T * >( args.bucket_box ) + static_cast< size_t >( r0 / kLeafSize ) * C;
+    for ( int k = lane; k < nb * D; k += 32 )
+    {
+      const int q = k / D, a = k - q * D;
+      T *col = s_el + q * kLeafSize * C + 2 * a;
+      T lo, hi;
+      io::load2( col, lo, hi );
+      if ( rows >= ( q + 1 ) * kLeafSize )
+      {
+#pragma unroll
+        for ( int j = 1; j < kLeafSize; ++j )
+        {
+          T l, h;
+          io::load2( col + j * C, l, h );
+          lo = io::mn( lo, l );
+          hi = io::mx( hi, h );
+        }
+      } else {
+        for ( int j = 1; j < rows - q * kLeafSize; ++j )
+        {
+          T l, h;
+          io::load2( col + j * C, l, h );
+          lo = io::mn( lo, l );
+          hi = io::mx( hi, h );
+        }
+      }
+      io::store2( col, lo, hi );
+      io::store2( bb + 2 * k, lo, hi );
+    }
+    __syncwarp();
+    // the group's union
+    if ( lane < D )
+    {
+      T lo, hi;
+      io::load2( s_el + 2 * lane, lo, hi );
+#pragma unroll
+      for ( int j = 1; j < G; ++j )
+        if ( j < nb )
+        {
+          T l, h;
+          io::load2( s_el + j * kLeafSize * C + 2 * lane, l, h );
+          lo = io::mn( lo, l );
+          hi = io::mx( hi, h );
+        }
+      io::store2( static_cast< T * >( args.warp_box ) + static_cast< size_t >( g ) * C + 2 * lane, lo, hi );
+      if ( n <= kLeafSize )
+      {
+        // one bucket: it is the tree
+        io::store2( reinterpret_cast< T * >( sc->root_box ) + 2 * lane, lo, hi );
+        if ( lane == 0 ) sc->root = ~0;
       }
     }
-#pragma unroll
-    for ( int a = 0; a < D; ++a )
-    {
-      s_el[tid * P + 2 * a] = lo[a];
-      s_el[tid * P + 2 * a + 1] = hi[a];
-    }
+    __syncwarp();
   }
-  __syncthreads();
-  if ( elem_rows )
-  {
-    // slab-major per leaf bucket: [bucket][slab][element j < 8][min, max], so the 8 elements' values of one slab are
-    // contiguous (the dense traversal reads them 8 lanes at a time)
-    T *eb = elem_rows + static_cast< size_t >( r0 ) * C;
-    const int nbk = ( rows + kLeafSize - 1 ) / kLeafSize;
-    for ( int k = tid; k < nbk * kLeafSize * C; k += kSlabThreads )
-    {
-      const int lb = k / ( kLeafSize * C ), rem = k - lb * ( kLeafSize * C );
-      const int a = rem / ( 2 * kLeafSize ), j = ( rem >> 1 ) & ( kLeafSize - 1 ), side = rem & 1;
-      const int q = lb * kLeafSize + j;
-      if ( q < rows ) eb[k] = s_el[q * P + 2 * a + side];
-    }
-  }
-  // bucket unions (ranks in order, as the serial union of the reference merges them)
-  const int nb = ( rows + kLeafSize - 1 ) / kLeafSize;
-  T *bb = bucket_box + static_cast< size_t >( r0 / kLeafSize ) * C;
-  for ( int k = tid; k < nb * C; k += kSlabThreads )
-  {
-    const int q = k / C, c = k - q * C;
-    const int j1 = min( kLeafSize, rows - q * kLeafSize );
-    T v = s_el[q * kLeafSize * P + c];
-    for ( int j = 1; j < j1; ++j )
-    {
-      const T x = s_el[( q * kLeafSize + j ) * P + c];
-      v = ( c & 1 ) ? io::mx( v, x ) : io::mn( v, x );
-    }
-    s_bk[q * P + c] = v;
-    bb[k] = v;
-  }
-  __syncthreads();
-  // query-group unions
-  const int ng = ( nb + G - 1 ) / G;
-  T *wb = warp_box + static_cast< size_t >( r0 / 32 ) * C;
-  for ( int k = tid; k < ng * C; k += kSlabThreads )
-  {
-    const int g = k / C, c = k - g * C;
-    const int j1 = min( G, nb - g * G );
-    T v = s_bk[g * G * P + c];
-    for ( int j = 1; j < j1; ++j )
-    {
-      const T x = s_bk[( g * G + j ) * P + c];
-      v = ( c & 1 ) ? io::mx( v, x ) : io::mn( v, x );
-    }
-    wb[k] = v;
-  }
-  if ( n <= kLeafSize )
-  {
-    // one bucket: it is the tree
-    T *rb = reinterpret_cast< T * >( sc->root_box );
-    if ( tid < C ) rb[tid] = s_bk[tid];
-    if ( tid == 0 ) sc->root = ~0;
-  }
+  if ( bad ) atomicCAS( &sc->error, 0, kErrTimeout );
 }
 
 // Phase 1 (one thread per leaf bucket b, blocks of 128 consecutive buckets).
@@ -875,20 +1012,53 @@ __device__ void refit_body(const tree_args &args, uint32_t bid, uint32_t)
   if ( mine && B0 + tid != root && !is_local( s_up[tid] >> 1 ) ) climb_from( s_up[tid], s_rng[tid].x - B0 );
 }
 
-uint32_t slab_grid(uint64_t n) { return static_cast< uint32_t >( ( n + kSlabThreads - 1 ) / kSlabThreads ); }
+template< int K, typename T, int VT >
+struct slab_kernels
+{
+  static constexpr int smem = kSlabSmem< K, T, VT >;
+  // Blocks of one object's launch: one warp per group of 32 ranks, at most the resident blocks (a persistent grid).
+  static uint32_t grid(uint64_t n)
+  {
+    const uint64_t want = ( n + 32 * kSlabWarps - 1 ) / ( 32 * kSlabWarps );
+    const uint64_t cap = static_cast< uint64_t >( device_sm_count() ) * kSlabBlocks< K, T, VT >;
+    return static_cast< uint32_t >( want < cap ? want : cap );
+  }
+  static cudaError_t setup()
+  {
+    if constexpr ( smem <= 47 * 1024 ) return cudaSuccess;
+    static std::atomic< unsigned long long > configured{ 0 };
+    int dev = 0;
+    cudaError_t e = cudaGetDevice( &dev );
+    if ( e != cudaSuccess ) return e;
+    const unsigned long long bit = 1ull << ( dev & 63 );
+    if ( configured.load() & bit ) return cudaSuccess;
+    e = cudaFuncSetAttribute( k_single< slabs_args, slabs_body< K, T, VT >, kSlabThreads, kSlabBlocks< K, T, VT > >,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
+    if ( e == cudaSuccess )
+      e = cudaFuncSetAttribute( k_batched< slabs_args, slabs_body< K, T, VT >, kSlabThreads, kSlabBlocks< K, T, VT > >,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
+    if ( e == cudaSuccess ) configured.fetch_or( bit );
+    return e;
+  }
+};
 
 template< int K, typename T, int VT >
 cudaError_t launch_slabs_t(const slabs_args &a, cudaStream_t s)
 {
-  k_single< slabs_args, slabs_body< K, T, VT >, kSlabThreads, kSlabMinBlocks< K, VT > ><<< slab_grid( a.n ), kSlabThreads, 0, s >>>( a );
+  const cudaError_t e = slab_kernels< K, T, VT >::setup();
+  if ( e != cudaSuccess ) return e;
+  k_single< slabs_args, slabs_body< K, T, VT >, kSlabThreads, kSlabBlocks< K, T, VT > >
+    <<< slab_kernels< K, T, VT >::grid( a.n ), kSlabThreads, kSlabSmem< K, T, VT >, s >>>( a );
   return cudaGetLastError();
 }
 
 template< int K, typename T, int VT >
 cudaError_t launch_slabs_batch_t(const batch_launch &b, cudaStream_t s)
 {
-  k_batched< slabs_args, slabs_body< K, T, VT >, kSlabThreads, kSlabMinBlocks< K, VT > ><<< b.blocks, kSlabThreads, 0, s >>>(
-    static_cast< const slabs_args * >( b.items ), b.starts, b.nitems );
+  const cudaError_t e = slab_kernels< K, T, VT >::setup();
+  if ( e != cudaSuccess ) return e;
+  k_batched< slabs_args, slabs_body< K, T, VT >, kSlabThreads, kSlabBlocks< K, T, VT > >
+    <<< b.blocks, kSlabThreads, kSlabSmem< K, T, VT >, s >>>( static_cast< const slabs_args * >( b.items ), b.starts, b.nitems );
   return cudaGetLastError();
 }
 
@@ -913,6 +1083,18 @@ cudaError_t slabs_batch_v(uint32_t V, const batch_launch &b, cudaStream_t s)
     case 4: return launch_slabs_batch_t< K, T, 4 >( b, s );
     case 8: return launch_slabs_batch_t< K, T, 8 >( b, s );
     default: return launch_slabs_batch_t< K, T, 0 >( b, s );
+  }
+}
+
+template< int K, typename T >
+uint32_t slabs_grid_v(uint32_t V, uint64_t n)
+{
+  switch ( V )
+  {
+    case 3: return slab_kernels< K, T, 3 >::grid( n );
+    case 4: return slab_kernels< K, T, 4 >::grid( n );
+    case 8: return slab_kernels< K, T, 8 >::grid( n );
+    default: return slab_kernels< K, T, 0 >::grid( n );
   }
 }
 
@@ -1054,7 +1236,19 @@ cudaError_t launch_slabs(int K, bool fp32, const double *verts, uint32_t V, uint
 #undef D
 }
 
-uint32_t slabs_blocks(uint64_t n) { return slab_grid( n ); }
+uint32_t slabs_blocks(int K, bool fp32, uint32_t V, uint64_t n)
+{
+#define F( KK ) slabs_grid_v< KK, float >( V, n )
+#define D( KK ) slabs_grid_v< KK, double >( V, n )
+  switch ( K )
+  {
+    case 6: return fp32 ? F( 6 ) : D( 6 );
+    case 18: return fp32 ? F( 18 ) : D( 18 );
+    default: return fp32 ? F( 26 ) : D( 26 );
+  }
+#undef F
+#undef D
+}
 
 cudaError_t launch_slabs_batch(int K, bool fp32, uint32_t V, const batch_launch &b, cudaStream_t s)
 {

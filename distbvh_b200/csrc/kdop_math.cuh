@@ -374,6 +374,65 @@ __device__ __forceinline__ void slabs32_all(const double *p, float eps_hi, float
   }
 }
 
+// FP64 slabs of group G's normals into the row (min, max per slab), in value those of slab64 (see project_group).
+template< int K, int G, int V >
+__device__ __forceinline__ void group_slabs64(const double *p, double eps, double *row)
+{
+  constexpr int N = group_size< G >;
+  constexpr int A0 = G == 0 ? 0 : ( G == 1 ? ( K == 18 ? 3 : 7 ) : 3 );  // the group's first normal
+  double lo[N], hi[N];
+#pragma unroll
+  for ( int v = 0; v < V; ++v )
+  {
+    double t[N];
+    project_group< G >( p[3 * v], p[3 * v + 1], p[3 * v + 2], t );
+#pragma unroll
+    for ( int k = 0; k < N; ++k )
+    {
+      lo[k] = v ? std_min( lo[k], t[k] ) : t[k];
+      hi[k] = v ? std_max( hi[k], t[k] ) : t[k];
+    }
+  }
+#pragma unroll
+  for ( int k = 0; k < N; ++k )
+  {
+    *reinterpret_cast< double2 * >( row + 2 * ( A0 + k ) ) = make_double2( __dsub_rn( lo[k], eps ), __dadd_rn( hi[k], eps ) );
+  }
+}
+
+// Slabs of an element from its V vertices in registers, (min, max) per slab into a row aligned to such a pair.
+template< int K, typename T, int V >
+__device__ __forceinline__ void vertex_slabs(const double *p, double eps, float eps_hi, T *row)
+{
+  constexpr int D = K / 2;
+  if constexpr ( sizeof( T ) == 8 )
+  {
+    // Non-finite coordinates (which only a refit can meet) take the reference's operation order.
+    unsigned most = 0;
+#pragma unroll
+    for ( int k = 0; k < V * 3; ++k ) most = max( most, static_cast< unsigned >( __double2hiint( p[k] ) ) & 0x7ff00000u );
+    if ( most != 0x7ff00000u )
+    {
+      group_slabs64< K, 0, V >( p, eps, row );
+      if constexpr ( K == 26 ) group_slabs64< K, 2, V >( p, eps, row );
+      if constexpr ( K >= 18 ) group_slabs64< K, 1, V >( p, eps, row );
+      return;
+    }
+#pragma unroll 1
+    for ( int a = 0; a < D; ++a )
+    {
+      double l, h;
+      slab64< K >( p, V, a, eps, l, h );
+      *reinterpret_cast< double2 * >( row + 2 * a ) = make_double2( l, h );
+    }
+  } else {
+    float lo[D], hi[D];
+    slabs32_all< K, V >( p, eps_hi, lo, hi );
+#pragma unroll
+    for ( int a = 0; a < D; ++a ) *reinterpret_cast< float2 * >( row + 2 * a ) = make_float2( lo[a], hi[a] );
+  }
+}
+
 // Slabs of element e (gathered vertices) into lo/hi.
 template< int K, typename T, int VT >
 __device__ __forceinline__ void leaf_slabs(const double *__restrict__ verts, uint32_t Vrt, uint32_t e, double eps,
