@@ -50,8 +50,8 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t *s
 // Persistent radix pass. A block keeps taking tiles from the pass's tile counter; while it ranks, resolves and
 // writes one tile, the next one is already streaming into the other half of its double-buffered shared memory
 // (TMA bulk copies on an mbarrier). Per tile: keys and indices to registers, stable warp-level ranking (the lanes
-// holding one digit meet by match; their leader takes the group's slots with one shared-memory atomic, which
-// retire in program order within the warp, and hands the base back by shuffle), per-digit tile counts published
+// holding one digit meet by match or by votes; their leader takes the group's slots with one shared-memory atomic,
+// which retire in program order within the warp, and hands the base back by shuffle), per-digit tile counts published
 // for the decoupled look-back, the tile reordered in the shared buffer it came from, contiguous digit runs
 // written out. Every wait is bounded (look-back polls and mbarrier waits); on a timeout the block raises the
 // object's error word and stops, and blocks that may have read a garbage prefix write only inside the output.
@@ -95,7 +95,14 @@ __device__ void onesweep_body(const sort_pass_args &a, uint32_t, uint32_t)
   auto stage_vals = [&](int st) { return reinterpret_cast< uint32_t * >( s_raw + st * kSortTile * 12 + kSortTile * 8 ); };
 
   // global exclusive offsets of the digits (the same for every tile of the pass)
-  const uint32_t gexcl = block_exclusive_scan( ( tid < RADIX ) ? hist[tid] : 0u, s_scan );
+  const uint32_t digits = ( tid < RADIX ) ? hist[tid] : 0u;
+  const uint32_t gexcl = block_exclusive_scan( digits, s_scan );
+  // How the lanes of a warp that hold one digit find each other: match costs more the more digits meet in a warp, one
+  // vote per digit bit costs the same for all. The line lies at 64 of 256 digits present in the pass. Two objects of
+  // 8.4M tetrahedra sort in 0.76 ms instead of 0.82, 2.1M each in 0.24 instead of 0.28 ms, a sphere of 1.3M triangles
+  // pass by pass in 22 us instead of 29 (its last, coherent pass in 22 instead of 19); the keys of a flat plate, a third
+  // of whose bits are constant, take 10% less with match.
+  const bool many = __syncthreads_count( digits != 0u ) > RADIX / 4;
   if ( tid == 0 )
   {
     mbar_init( &s_mbar[0], 1 );
@@ -177,8 +184,22 @@ __device__ void onesweep_body(const sort_pass_args &a, uint32_t, uint32_t)
     {
       const bool valid = ( wl + j * 32 + lane ) < cnt;
       const uint32_t d = valid ? digit( k[j] ) : RADIX;
-      const unsigned peers = __match_any_sync( 0xffffffffu, d );
-      const int leader = __ffs( peers ) - 1;
+      // the lanes that hold this lane's digit
+      unsigned peers;
+      if ( many )
+      {
+        peers = __ballot_sync( 0xffffffffu, valid );
+#pragma unroll
+        for ( int bit = 0; bit < BITS; ++bit )
+        {
+          const bool one = ( d >> bit ) & 1u;
+          const unsigned v = __ballot_sync( 0xffffffffu, one );
+          peers &= one ? v : ~v;
+        }
+      } else {
+        peers = __match_any_sync( 0xffffffffu, d );
+      }
+      const int leader = valid ? __ffs( peers ) - 1 : lane;
       uint32_t base = 0;
       if ( valid && lane == leader )
         base = ( atomicAdd( &s_whist[wrow][d], static_cast< uint32_t >( __popc( peers ) ) << wsh ) >> wsh ) & 0xffffu;
