@@ -412,7 +412,8 @@ struct recheck_args
   uint64_t cap;
   pair_scalars *ps;
 };
-uint32_t recheck_blocks(uint64_t ncand);
+// The scenes' rechecks, and below their id outputs, in one launch each over the resident blocks (items only: the
+// scenes' counts divide the work on the device).
 cudaError_t launch_recheck_batch(int K, uint32_t V, const batch_launch &b, cudaStream_t s);
 
 struct gid_args
@@ -425,7 +426,6 @@ struct gid_args
   int normalize;
   uint64_t *out;
 };
-uint32_t gid_pairs_dev_blocks(uint64_t cap);
 cudaError_t launch_gid_pairs_dev_batch(const batch_launch &b, cudaStream_t s);
 
 // Queries every leaf of q against tree t; writes (q element, t element) local index pairs. dense (both objects'

@@ -828,11 +828,18 @@ __device__ __forceinline__ void load_verts(const double *p, bool vec16, double *
 constexpr int kRecheckThreads = 256;
 constexpr int kRecheckBuf = 128;  // buffered pairs per warp: drained once more than 96 are held
 
+// The candidate count is read on the device: no host round trip between traversal and recheck.
+__device__ __forceinline__ uint64_t candidates(const recheck_args &args)
+{
+  return min( static_cast< uint64_t >( *reinterpret_cast< volatile unsigned long long * >( &args.ps->count ) ), args.cand_cap );
+}
+
 // K7: FP64 overlap of both elements from their vertices. With both vertex counts known at compile time, the
 // comparison-only projections of overlap64 (shared products, no products by 0 or 1, one epsilon shift per slab);
 // otherwise slab64 slab by slab with early exit. Both give the outcome of comparing the FP64 slabs.
+// One warp takes the groups of 32 candidates u0, u0 + step, ... below u1; wout: its pair buffer.
 template< int K, int VA, int VB >
-__device__ void recheck_body(const recheck_args &args, uint32_t bid, uint32_t nblk)
+__device__ __forceinline__ void recheck_groups(const recheck_args &args, uint64_t u0, uint64_t u1, uint64_t step, uint2 *wout)
 {
   const double *__restrict__ va = args.va;
   const uint32_t Var = args.Va;
@@ -840,23 +847,18 @@ __device__ void recheck_body(const recheck_args &args, uint32_t bid, uint32_t nb
   const uint32_t Vbr = args.Vb;
   const double eps = args.eps;
   const uint2 *__restrict__ cand = args.cand;
-  const uint64_t cand_cap = args.cand_cap;
   uint2 *out = args.out;
   const uint64_t cap = args.cap;
   pair_scalars *ps = args.ps;
   constexpr int D = K / 2;
-  // The candidate count is read on the device: no host round trip between traversal and recheck.
-  const uint64_t ncand = min( static_cast< uint64_t >( *reinterpret_cast< volatile unsigned long long * >( &ps->count ) ),
-                              cand_cap );
+  const uint64_t ncand = candidates( args );
   const int Va = VA > 0 ? VA : static_cast< int >( Var );
   const int Vb = VB > 0 ? VB : static_cast< int >( Vbr );
   const bool vec16 = ( ( reinterpret_cast< uintptr_t >( va ) | reinterpret_cast< uintptr_t >( vb ) ) & 15 ) == 0;
   // Confirmed pairs collect in a per-warp buffer in shared memory and leave through one atomic reservation per
   // 97-128 pairs, with coalesced stores (one same-address atomic per 32 candidates made the kernel wait on the
   // counter's round trip).
-  __shared__ uint2 s_out[kRecheckThreads / 32][kRecheckBuf];
   const unsigned lane = threadIdx.x & 31u, lt = ( 1u << lane ) - 1u;
-  uint2 *wout = s_out[threadIdx.x >> 5];
   uint32_t nout = 0;
   auto drain = [&]() {
     __syncwarp();
@@ -868,11 +870,9 @@ __device__ void recheck_body(const recheck_args &args, uint32_t bid, uint32_t nb
     __syncwarp();
     nout = 0;
   };
-  // warp-uniform trips: lane l of a warp takes candidate p0 + l
-  for ( uint64_t p0 = static_cast< uint64_t >( bid ) * blockDim.x + ( threadIdx.x & ~31u ); p0 < ncand;
-        p0 += static_cast< uint64_t >( nblk ) * blockDim.x )
+  for ( uint64_t u = u0; u < u1; u += step )
   {
-    const uint64_t p = p0 + lane;
+    const uint64_t p = 32 * u + lane;
     const bool valid = p < ncand;
     const uint2 c = valid ? __ldg( cand + p ) : make_uint2( 0u, 0u );
     bool ok = valid;
@@ -922,6 +922,85 @@ __device__ void recheck_body(const recheck_args &args, uint32_t bid, uint32_t nb
   drain();
 }
 
+template< int K, int VA, int VB >
+__device__ void recheck_body(const recheck_args &args, uint32_t bid, uint32_t nblk)
+{
+  __shared__ uint2 s_out[kRecheckThreads / 32][kRecheckBuf];
+  constexpr uint32_t W = kRecheckThreads / 32;
+  recheck_groups< K, VA, VB >( args, static_cast< uint64_t >( bid ) * W + ( threadIdx.x >> 5 ), ( candidates( args ) + 31 ) / 32,
+                               static_cast< uint64_t >( nblk ) * W, s_out[threadIdx.x >> 5] );
+}
+
+// ---- the scenes of a batch in one launch ----------------------------------------------------------------------
+//
+// Each scene's pair count is known on the device only, and most scenes of a batch have few or none: a launch with
+// blocks for every scene's capacity spends its time on starting blocks that find nothing (496 pairs of 32 bodies, most
+// of them apart: 294,000 blocks, 1.0 ms for the recheck and 0.24 ms for the ids over the groups of a batch). A grid of
+// the resident blocks instead forms the running sum of the scenes' counts, kSceneTile scenes at a time, and divides the
+// sum.
+constexpr int kSceneTile = 2 * kRecheckThreads;
+
+// pre[0 .. count] = the exclusive running sum of f(0 .. count - 1), by a block of kRecheckThreads threads.
+template< typename F >
+__device__ __forceinline__ void scene_sum(int count, F f, unsigned long long *pre)
+{
+  __shared__ unsigned long long s_warp[kRecheckThreads / 32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const unsigned long long v0 = 2 * t < count ? f( 2 * t ) : 0ull, v1 = 2 * t + 1 < count ? f( 2 * t + 1 ) : 0ull;
+  unsigned long long inc = v0 + v1;
+#pragma unroll
+  for ( int o = 1; o < 32; o <<= 1 )
+  {
+    const unsigned long long y = __shfl_up_sync( 0xffffffffu, inc, o );
+    if ( lane >= o ) inc += y;
+  }
+  if ( lane == 31 ) s_warp[w] = inc;
+  __syncthreads();
+  for ( int k = 0; k < w; ++k ) inc += s_warp[k];
+  if ( t == 0 ) pre[0] = 0ull;
+  if ( 2 * t < count ) pre[2 * t + 1] = inc - v1;
+  if ( 2 * t + 1 < count ) pre[2 * t + 2] = inc;
+  __syncthreads();
+}
+
+// The last scene whose sum is <= u (u below the total).
+__device__ __forceinline__ int scene_of(const unsigned long long *pre, int count, unsigned long long u)
+{
+  int lo = 0, hi = count - 1;
+  while ( lo < hi )
+  {
+    const int mid = ( lo + hi + 1 ) >> 1;
+    if ( pre[mid] <= u ) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// The recheck of n scenes: every warp takes an equal share of consecutive groups of 32 candidates.
+template< int K, int VA, int VB >
+__global__ void __launch_bounds__( kRecheckThreads, 2 ) k_recheck_scenes(const recheck_args *__restrict__ items, int n)
+{
+  constexpr uint32_t W = kRecheckThreads / 32;
+  __shared__ uint2 s_out[W][kRecheckBuf];
+  __shared__ unsigned long long s_pre[kSceneTile + 1];
+  const unsigned long long warps = static_cast< unsigned long long >( gridDim.x ) * W, w = blockIdx.x * W + ( threadIdx.x >> 5 );
+  for ( int t0 = 0; t0 < n; t0 += kSceneTile )
+  {
+    const int count = min( kSceneTile, n - t0 );
+    scene_sum( count, [&](int s) -> unsigned long long { return ( candidates( items[t0 + s] ) + 31 ) / 32; }, s_pre );
+    const unsigned long long total = s_pre[count], end = total * ( w + 1 ) / warps;
+    for ( unsigned long long u = total * w / warps; u < end; )
+    {
+      const int s = scene_of( s_pre, count, u );
+      const unsigned long long last = min( end, s_pre[s + 1] );
+      const recheck_args a = items[t0 + s];
+      recheck_groups< K, VA, VB >( a, u - s_pre[s], last - s_pre[s], 1, s_out[threadIdx.x >> 5] );
+      u = last;
+    }
+    __syncthreads();  // the next tile reuses the sums
+  }
+}
+
 // grid-stride over the candidates (their count is read on the device): at most 4 blocks per SM
 uint32_t recheck_grid(uint64_t ncand)
 {
@@ -945,10 +1024,11 @@ template< int K >
 cudaError_t recheck_batch_k(uint32_t V, const batch_launch &b, cudaStream_t s)
 {
   const recheck_args *it = static_cast< const recheck_args * >( b.items );
-  if ( V == 3 ) k_batched< recheck_args, recheck_body< K, 3, 3 >, kRecheckThreads, 2 ><<< b.blocks, kRecheckThreads, 0, s >>>( it, b.starts, b.nitems );
-  else if ( V == 4 ) k_batched< recheck_args, recheck_body< K, 4, 4 >, kRecheckThreads, 2 ><<< b.blocks, kRecheckThreads, 0, s >>>( it, b.starts, b.nitems );
-  else if ( V == 8 ) k_batched< recheck_args, recheck_body< K, 8, 8 >, kRecheckThreads, 2 ><<< b.blocks, kRecheckThreads, 0, s >>>( it, b.starts, b.nitems );
-  else k_batched< recheck_args, recheck_body< K, 0, 0 >, kRecheckThreads, 2 ><<< b.blocks, kRecheckThreads, 0, s >>>( it, b.starts, b.nitems );
+  const uint32_t grid = static_cast< uint32_t >( device_sm_count() ) * 2;
+  if ( V == 3 ) k_recheck_scenes< K, 3, 3 ><<< grid, kRecheckThreads, 0, s >>>( it, b.nitems );
+  else if ( V == 4 ) k_recheck_scenes< K, 4, 4 ><<< grid, kRecheckThreads, 0, s >>>( it, b.nitems );
+  else if ( V == 8 ) k_recheck_scenes< K, 8, 8 ><<< grid, kRecheckThreads, 0, s >>>( it, b.nitems );
+  else k_recheck_scenes< K, 0, 0 ><<< grid, kRecheckThreads, 0, s >>>( it, b.nitems );
   return cudaGetLastError();
 }
 
@@ -968,18 +1048,44 @@ __global__ void k_gid_pairs(const uint2 *__restrict__ pairs, uint64_t count, con
 
 // k_gid_pairs with the count read on the device (at most cap): for launches whose count is unknown when they are
 // enqueued (batched scenes in a CUDA graph).
+__device__ __forceinline__ uint64_t gid_count(const gid_args &a)
+{
+  return min( static_cast< uint64_t >( *reinterpret_cast< const volatile unsigned long long * >( a.count ) ), a.cap );
+}
+
+__device__ __forceinline__ void write_ids(const gid_args &a, uint64_t p)
+{
+  uint2 c = a.pairs[p];
+  if ( a.normalize && c.x > c.y ) c = make_uint2( c.y, c.x );
+  const uint64_t ga = a.gid_a ? __ldg( a.gid_a + c.x ) : c.x;
+  const uint64_t gb = a.gid_b ? __ldg( a.gid_b + c.y ) : c.y;
+  reinterpret_cast< ulonglong2 * >( a.out )[p] = make_ulonglong2( ga, gb );
+}
+
 __device__ void gid_dev_body(const gid_args &a, uint32_t bid, uint32_t nblk)
 {
-  const uint64_t n = min( static_cast< uint64_t >( *reinterpret_cast< const volatile unsigned long long * >( a.count ) ),
-                          a.cap );
+  const uint64_t n = gid_count( a );
   for ( uint64_t p = static_cast< uint64_t >( bid ) * blockDim.x + threadIdx.x; p < n;
         p += static_cast< uint64_t >( nblk ) * blockDim.x )
+    write_ids( a, p );
+}
+
+// The same for n scenes in one launch (see "the scenes of a batch in one launch").
+__global__ void __launch_bounds__( kRecheckThreads ) k_gid_scenes(const gid_args *__restrict__ items, int n)
+{
+  __shared__ unsigned long long s_pre[kSceneTile + 1];
+  for ( int t0 = 0; t0 < n; t0 += kSceneTile )
   {
-    uint2 c = a.pairs[p];
-    if ( a.normalize && c.x > c.y ) c = make_uint2( c.y, c.x );
-    const uint64_t ga = a.gid_a ? __ldg( a.gid_a + c.x ) : c.x;
-    const uint64_t gb = a.gid_b ? __ldg( a.gid_b + c.y ) : c.y;
-    reinterpret_cast< ulonglong2 * >( a.out )[p] = make_ulonglong2( ga, gb );
+    const int count = min( kSceneTile, n - t0 );
+    scene_sum( count, [&](int s) -> unsigned long long { return gid_count( items[t0 + s] ); }, s_pre );
+    const unsigned long long total = s_pre[count];
+    for ( unsigned long long u = static_cast< unsigned long long >( blockIdx.x ) * kRecheckThreads + threadIdx.x; u < total;
+          u += static_cast< unsigned long long >( gridDim.x ) * kRecheckThreads )
+    {
+      const int s = scene_of( s_pre, count, u );
+      write_ids( items[t0 + s], u - s_pre[s] );
+    }
+    __syncthreads();  // the next tile reuses the sums
   }
 }
 
@@ -992,7 +1098,7 @@ __global__ void k_gather_words(const int *const *__restrict__ src, int n, int *_
 
 }  // namespace
 
-uint32_t gid_pairs_dev_blocks(uint64_t cap)
+static uint32_t gid_pairs_dev_blocks(uint64_t cap)
 {
   const uint64_t blocks = ( cap + 255 ) / 256;
   return static_cast< uint32_t >( blocks < 148 * 2 ? ( blocks ? blocks : 1 ) : 148 * 2 );
@@ -1011,8 +1117,8 @@ cudaError_t launch_gid_pairs_dev(const uint2 *pairs, const unsigned long long *c
 cudaError_t launch_gid_pairs_dev_batch(const batch_launch &b, cudaStream_t s)
 {
   if ( !b.nitems ) return cudaSuccess;
-  k_batched< gid_args, gid_dev_body, 256, 1 ><<< b.blocks, 256, 0, s >>>( static_cast< const gid_args * >( b.items ),
-                                                                        b.starts, b.nitems );
+  k_gid_scenes<<< static_cast< uint32_t >( device_sm_count() ) * 2, kRecheckThreads, 0, s >>>( static_cast< const gid_args * >( b.items ),
+                                                                                             b.nitems );
   return cudaGetLastError();
 }
 
@@ -1051,8 +1157,6 @@ cudaError_t launch_recheck(int K, const double *verts_a, uint32_t Va, const doub
     default: return cudaErrorInvalidValue;
   }
 }
-
-uint32_t recheck_blocks(uint64_t ncand) { return recheck_grid( ncand ); }
 
 cudaError_t launch_recheck_batch(int K, uint32_t V, const batch_launch &b, cudaStream_t s)
 {
