@@ -39,11 +39,41 @@ __global__ void __launch_bounds__( THREADS, MIN_BLOCKS ) k_batched(const Args *_
   Body( a, blockIdx.x - b0, __ldg( starts + i + 1 ) - b0 );
 }
 
-// One per-object launch of a body.
+// One per-object launch of a body. An object's kernels follow one another in a stream, each reading what the last one
+// wrote. For a small object launch_chained() lets the next kernel's blocks start while this one's still run, and every
+// kernel waits here until the kernels before it have completed and their writes are visible (so a chain of waiting
+// kernels is ordered as a plain one). What overlaps is the launch itself: the 12 kernels of a build of 10,000 triangles
+// take a few microseconds each, and a step of two such objects went from 412 to 381 us, one of 200,003 tetrahedra from
+// 467 to 458 us, two blocks of 512 hexahedra from 356 to 345 us. Above kChainElements the launches are plain: there the
+// waiting blocks take the place of the other object's kernels (1.3M and 1.0M triangles 526 -> 554 us with the chain, a
+// refit of 9.4M triangles 682 -> 713 us).
+constexpr uint64_t kChainElements = 1u << 19;
+constexpr uint32_t kChainBlocks = 296;  // a grid beyond it fills the device: its successor starts after it
+
 template< typename Args, void ( *Body )( const Args &, uint32_t, uint32_t ), int THREADS, int MIN_BLOCKS >
 __global__ void __launch_bounds__( THREADS, MIN_BLOCKS ) k_single(const Args a)
 {
+  if ( gridDim.x <= kChainBlocks ) asm volatile( "griddepcontrol.launch_dependents;" ::: "memory" );
+  asm volatile( "griddepcontrol.wait;" ::: "memory" );
   Body( a, blockIdx.x, gridDim.x );
+}
+
+// Launches a per-object kernel whose predecessor in the stream is the previous kernel of the object (n elements).
+template< typename Args >
+cudaError_t launch_chained(uint64_t n, void ( *kernel )( Args ), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t s,
+                           const Args &a)
+{
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3( grid );
+  cfg.blockDim = dim3( threads );
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = n <= kChainElements ? 1 : 0;
+  return cudaLaunchKernelEx( &cfg, kernel, a );
 }
 
 // Host side: a batched launch description (item arguments and block starts on the device, built when a batch graph

@@ -418,15 +418,14 @@ cudaError_t launch_cb_t(const cb_args &a, cudaStream_t s)
       int per_sm = 1;
       cudaError_t e = cb_tma_setup< K, VT >( &per_sm );
       if ( e != cudaSuccess ) return e;
-      k_single< cb_args, cb_tma_body< K, VT >, kElemThreads, kCbTmaMinBlocks< K, VT > >
-        <<< cb_grid( a.n, true, per_sm ), kElemThreads, cb_smem( VT, true ), s >>>( a );
-      return cudaGetLastError();
+      return launch_chained( a.n, k_single< cb_args, cb_tma_body< K, VT >, kElemThreads, kCbTmaMinBlocks< K, VT > >,
+                             cb_grid( a.n, true, per_sm ), kElemThreads, cb_smem( VT, true ), s, a );
     }
   }
   cudaError_t e = cb_plain_setup< K, VT >( a.V );
   if ( e != cudaSuccess ) return e;
-  k_single< cb_args, cb_body< K, VT >, kElemThreads, 4 ><<< cb_grid( a.n, false, 0 ), kElemThreads, cb_smem( a.V, false ), s >>>( a );
-  return cudaGetLastError();
+  return launch_chained( a.n, k_single< cb_args, cb_body< K, VT >, kElemThreads, 4 >, cb_grid( a.n, false, 0 ), kElemThreads,
+                         cb_smem( a.V, false ), s, a );
 }
 
 // Batched: every item's verts 16-byte aligned and VT > 0 for the TMA form (tma), one V for all items.
@@ -487,8 +486,7 @@ uint32_t kh_grid(uint64_t n)
 template< int BITS >
 cudaError_t launch_kh_t(const kh_args &a, cudaStream_t s)
 {
-  k_single< kh_args, kh_body< BITS >, kElemThreads, 1 ><<< kh_grid( a.n ), kElemThreads, 0, s >>>( a );
-  return cudaGetLastError();
+  return launch_chained( a.n, k_single< kh_args, kh_body< BITS >, kElemThreads, 1 >, kh_grid( a.n ), kElemThreads, 0, s, a );
 }
 
 template< int BITS >

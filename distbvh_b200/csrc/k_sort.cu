@@ -377,8 +377,8 @@ cudaError_t launch_os_t(const sort_pass_args &a, cudaStream_t s)
 {
   cudaError_t e = onesweep_setup< BITS >();
   if ( e != cudaSuccess ) return e;
-  k_single< sort_pass_args, onesweep_body< BITS >, kSortThreads, 2 ><<< os_grid( a.n ), kSortThreads, kOnesweepSmem, s >>>( a );
-  return cudaGetLastError();
+  return launch_chained( a.n, k_single< sort_pass_args, onesweep_body< BITS >, kSortThreads, 2 >, os_grid( a.n ), kSortThreads,
+                         kOnesweepSmem, s, a );
 }
 
 template< int BITS >
@@ -641,9 +641,10 @@ cudaError_t launch_sort_fixup(const uint64_t *keys_in, const uint32_t *vals_in, 
 {
   if ( n == 0 ) return cudaSuccess;
   const fixup_args a{ keys_in, vals_in, keys_out, vals_out, n, runs, sc };
-  k_single< fixup_args, fixup_body, 256, 8 ><<< sort_fixup_blocks( n ), 256, 0, s >>>( a );
-  if ( const uint32_t rb = sort_runs_blocks( n ) ) k_single< fixup_args, runs_body, kFixThreads, 1 ><<< rb, kFixThreads, 0, s >>>( a );
-  return cudaGetLastError();
+  const cudaError_t e = launch_chained( a.n, k_single< fixup_args, fixup_body, 256, 8 >, sort_fixup_blocks( n ), 256, 0, s, a );
+  const uint32_t rb = sort_runs_blocks( n );
+  if ( e != cudaSuccess || !rb ) return e;
+  return launch_chained( a.n, k_single< fixup_args, runs_body, kFixThreads, 1 >, rb, kFixThreads, 0, s, a );
 }
 
 cudaError_t launch_sort_fixup_batch(const batch_launch &b, cudaStream_t s)

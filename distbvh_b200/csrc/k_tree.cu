@@ -1047,9 +1047,8 @@ cudaError_t launch_slabs_t(const slabs_args &a, cudaStream_t s)
 {
   const cudaError_t e = slab_kernels< K, T, VT >::setup();
   if ( e != cudaSuccess ) return e;
-  k_single< slabs_args, slabs_body< K, T, VT >, kSlabThreads, kSlabBlocks< K, T, VT > >
-    <<< slab_kernels< K, T, VT >::grid( a.n ), kSlabThreads, kSlabSmem< K, T, VT >, s >>>( a );
-  return cudaGetLastError();
+  return launch_chained( a.n, k_single< slabs_args, slabs_body< K, T, VT >, kSlabThreads, kSlabBlocks< K, T, VT > >,
+                         slab_kernels< K, T, VT >::grid( a.n ), kSlabThreads, kSlabSmem< K, T, VT >, s, a );
 }
 
 template< int K, typename T, int VT >
@@ -1124,8 +1123,8 @@ cudaError_t launch_build_t(const tree_args &a, cudaStream_t s)
   if ( !grid ) return cudaSuccess;  // the slab kernel stored a one-bucket object's root
   const cudaError_t e = build_setup< K, T >();
   if ( e != cudaSuccess ) return e;
-  k_single< tree_args, build_leaf_body< K, T >, kBuildThreads, 8 ><<< grid, kBuildThreads, kBuildSmem< K, T >, s >>>( a );
-  return cudaGetLastError();
+  return launch_chained( a.n, k_single< tree_args, build_leaf_body< K, T >, kBuildThreads, 8 >, grid, kBuildThreads,
+                         kBuildSmem< K, T >, s, a );
 }
 
 template< int K, typename T >
@@ -1149,8 +1148,7 @@ uint32_t climb_grid(uint64_t n)
 template< int K, typename T >
 cudaError_t launch_climb_t(const tree_args &a, cudaStream_t s)
 {
-  k_single< tree_args, climb_body< K, T >, 128, 4 ><<< climb_grid( a.n ), 128, 0, s >>>( a );
-  return cudaGetLastError();
+  return launch_chained( a.n, k_single< tree_args, climb_body< K, T >, 128, 4 >, climb_grid( a.n ), 128, 0, s, a );
 }
 
 template< int K, typename T >
@@ -1172,8 +1170,7 @@ cudaError_t launch_refit_t(const tree_args &a, cudaStream_t s)
 {
   const uint32_t grid = refit_grid( a.n );
   if ( !grid ) return cudaSuccess;
-  k_single< tree_args, refit_body< K, T >, kBuildThreads, 7 ><<< grid, kBuildThreads, 0, s >>>( a );
-  return cudaGetLastError();
+  return launch_chained( a.n, k_single< tree_args, refit_body< K, T >, kBuildThreads, 7 >, grid, kBuildThreads, 0, s, a );
 }
 
 template< int K, typename T >
