@@ -754,7 +754,7 @@ bvhg_status capture_batch(bvhg_ctx *ctx, batch_state &B, const batch_args &x, co
       if ( oa.n == 0 || ob.n == 0 || ( self && oa.n < 2 ) ) continue;
       uint2 *cand = B.cand.as< uint2 >() + B.off[sc];
       BVHG_CUDA( ctx, launch_traverse( K, fp32, view_of( oa ), view_of( ob ), self, oa.dense_ok && ob.dense_ok,
-                                       ctx->cfg.epsilon, cand, B.cap[sc], ps + sc, ls, ctx->dense_stack ) );
+                                       ctx->cfg.epsilon, cand, B.cap[sc], ps + sc, ls, ctx->dense_stack, false ) );
       const uint2 *fin = cand;
       const unsigned long long *cnt = &ps[sc].count;
       if ( fp32 )

@@ -388,6 +388,7 @@ struct trav_item
   uint64_t cap;
   pair_scalars *ps;
   int dense_stack;
+  uint32_t width;  // queries per packet of the walk over stored slabs
   const obj_scalars *qsc;
 };
 
@@ -431,9 +432,10 @@ cudaError_t launch_gid_pairs_dev_batch(const batch_launch &b, cudaStream_t s);
 // Queries every leaf of q against tree t; writes (q element, t element) local index pairs. dense (both objects'
 // element slabs stored): the walk that pops nodes in batches and tests leaves in batches; its deeper stack bound can
 // be reached (ps->error = kErrOverflowStack), and the single-node walk (dense = false) then always completes.
-// dense_stack_limit > 0 lowers that bound (test hook); 0 keeps it.
+// dense_stack_limit > 0 lowers that bound (test hook); 0 keeps it. alone: nothing else runs beside the search, so that a
+// small q may take packets of fewer queries (one scene of a batch shares the device).
 cudaError_t launch_traverse(int K, bool fp32, tree_view q, tree_view t, bool self, bool dense, double eps, uint2 *pairs,
-                            uint64_t cap, pair_scalars *ps, cudaStream_t s, int dense_stack_limit = 0);
+                            uint64_t cap, pair_scalars *ps, cudaStream_t s, int dense_stack_limit = 0, bool alone = true);
 
 // FP64 recheck of FP32 candidates: keeps (a, b) iff the FP64 slabs of a and b overlap, compacted into out.
 // The candidate count is min(ps->count, cand_cap), read on the device.

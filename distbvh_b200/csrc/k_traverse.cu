@@ -420,15 +420,16 @@ __device__ __forceinline__ void filter_buckets(const trav_args< T > &x, walk_sme
   __syncwarp();
 }
 
-// One packet: ranks i0 .. i0 + 31 against the target tree (see above). rb: the target root's slabs.
+// One packet: ranks i0 .. i0 + width - 1 (width 8 or 32) against the target tree (see above). rb: the target root's
+// slabs.
 template< int K, typename T, int VT, bool STORED >
-__device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint32_t i0, const unsigned lane,
-                                            walk_smem< K, T > &sm, const T *rb)
+__device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint32_t i0, const uint32_t width,
+                                            const unsigned lane, walk_smem< K, T > &sm, const T *rb)
 {
   constexpr int D = K / 2;
   const uint32_t i = i0 + lane;
   const T *wb = x.qwarp + static_cast< size_t >( i0 >> 5 ) * K;
-  // 1. The packet's union box against the target's root box (uniform over the warp).
+  // 1. The union box of the 32 ranks around the packet against the target's root box (uniform over the warp).
   {
     bool o = true;
 #pragma unroll
@@ -436,7 +437,7 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
     if ( !o ) return;
   }
   // 2. Each lane's own slabs (stored, or from its element's vertices) against the root box.
-  const bool valid = i < x.nq;
+  const bool valid = i < x.nq && lane < width;
   const uint32_t qe = valid ? __ldg( x.qperm + i ) : 0u;
   if constexpr ( STORED )
   {
@@ -449,8 +450,30 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
     if ( valid ) slabs_to_row< K, T, VT >( x.qverts, x.qV, qe, x.eps, x.eps_hi, sm.q[lane] );
   }
   sm.qe[lane] = qe;
-  if ( lane < K ) sm.g[lane] = __ldg( wb + lane );
-  __syncwarp();
+  if ( width == 32u )
+  {
+    if ( lane < K ) sm.g[lane] = __ldg( wb + lane );
+    __syncwarp();
+  } else {
+    __syncwarp();
+    if ( lane < D )
+    {
+      // the union of the packet's rows (lanes past them hold its first one)
+      T lo, hi;
+      shared_pair( &sm.q[0][2 * lane], lo, hi );
+      const uint32_t rows = min( width, x.nq - i0 );
+      for ( uint32_t j = 1; j < rows; ++j )
+      {
+        T l, h;
+        shared_pair( &sm.q[j][2 * lane], l, h );
+        lo = l < lo ? l : lo;
+        hi = hi < h ? h : hi;
+      }
+      sm.g[2 * lane] = lo;
+      sm.g[2 * lane + 1] = hi;
+    }
+    __syncwarp();
+  }
   bool in_root = valid;
 #pragma unroll
   for ( int a = 0; a < D; ++a )
@@ -651,7 +674,7 @@ __device__ void traverse_body(const trav_item &item, uint32_t, uint32_t)
     for ( unsigned m = __ballot_sync( 0xffffffffu, o ); m; m &= m - 1 )
     {
       const uint32_t p = c + static_cast< uint32_t >( __ffs( m ) - 1 ) * chunks;
-      walk_packet< K, T, VT, false >( x, p * 32, lane, sm, rb );
+      walk_packet< K, T, VT, false >( x, p * 32, 32u, lane, sm, rb );
     }
   }
 }
@@ -666,9 +689,9 @@ __device__ void stored_body(const trav_item &item, uint32_t bid, uint32_t)
   const unsigned lane = threadIdx.x & 31u;
   if ( !objects_meet< K, T >( x, item.qsc ) ) return;
   const T *rb = reinterpret_cast< const T * >( x.tsc->root_box );
-  const uint32_t packets = ( x.nq + 31 ) / 32;
+  const uint32_t width = item.width;
   const uint32_t pk = ( bid * blockDim.x + threadIdx.x ) >> 5;
-  if ( pk < packets ) walk_packet< K, T, 0, true >( x, pk * 32, lane, sm, rb );
+  if ( static_cast< uint64_t >( pk ) * width < x.nq ) walk_packet< K, T, 0, true >( x, pk * width, width, lane, sm, rb );
 }
 
 // Shared memory per block of the walks, and their resident blocks per SM: as many as it allows (228 KB per SM, 1 KB of
@@ -685,8 +708,16 @@ constexpr int kWalkBlocks = kWalkBySmem< K, T, STORED > < kWalkCap< K, T, STORED
 
 // One scene's item and grid. Dense contact: one warp per packet. Sparse: a persistent grid of at most the resident
 // blocks (4 per SM), one warp per chunk of 32 packets at most.
+//
+// Queries per packet in dense contact. A walk is a chain of steps: a small object whose packets of 32 do not fill the
+// device takes packets of one bucket (8), four times the warps with shorter chains. The line lies where those still run
+// at once (148 SMs x 16 warps): two plates of 1,600 / 10,000 triangles 64 / 91 -> 33 / 59 us, two blocks of 512 / 8,000
+// hexahedra 39 / 100 -> 22 / 54 us; beyond it the work of the narrow packets counts: 32,768 hexahedra 53 -> 64 us,
+// 70,000 tetrahedra against themselves 83 -> 113 us, and a batch, whose scenes share the device, 9.8 -> 13.3 ms.
+constexpr uint64_t kNarrowQueries = 148 * 16 * 8;
+
 template< int K, typename T >
-void trav_item_t(tree_view q, tree_view t, bool self, bool dense, double eps, uint2 *pairs, uint64_t cap,
+void trav_item_t(tree_view q, tree_view t, bool self, bool dense, bool alone, double eps, uint2 *pairs, uint64_t cap,
                  pair_scalars *ps, int dense_stack_limit, trav_item *it, uint32_t *blocks, bool *dense_out)
 {
   it->qwarp = q.warp_box;
@@ -713,11 +744,12 @@ void trav_item_t(tree_view q, tree_view t, bool self, bool dense, double eps, ui
   it->dense_stack = dense_stack_limit > 0 && dense_stack_limit < kWalkStack ? dense_stack_limit : kWalkStack;
   it->qsc = q.sc;
   constexpr uint64_t kWarps = kTravThreads / 32;
-  const uint64_t packets = ( q.n + 31 ) / 32;
-  const uint64_t chunks = ( packets + 31 ) / 32;
+  const uint64_t chunks = ( ( q.n + 31 ) / 32 + 31 ) / 32;
   const uint64_t resident = static_cast< uint64_t >( device_sm_count() ) * kTravBlocksPerSM;
   dense = dense && q.stored && t.stored;
-  uint64_t b = dense ? ( packets + kWarps - 1 ) / kWarps : ( chunks + kWarps - 1 ) / kWarps;
+  it->width = alone && q.n <= kNarrowQueries ? 8u : 32u;
+  const uint64_t width = it->width;
+  uint64_t b = dense ? ( ( q.n + width - 1 ) / width + kWarps - 1 ) / kWarps : ( chunks + kWarps - 1 ) / kWarps;
   if ( !dense && b > resident ) b = resident;
   *blocks = static_cast< uint32_t >( b < ( 1ull << 30 ) ? ( b ? b : 1 ) : ( 1ull << 30 ) );
   *dense_out = dense;
@@ -771,11 +803,11 @@ struct walk_kernels
 
 template< int K, typename T >
 cudaError_t launch_trav_t(tree_view q, tree_view t, bool self, bool dense, double eps, uint2 *pairs, uint64_t cap,
-                          pair_scalars *ps, cudaStream_t s, int dense_stack_limit)
+                          pair_scalars *ps, cudaStream_t s, int dense_stack_limit, bool alone)
 {
   trav_item it;
   uint32_t grid = 0;
-  trav_item_t< K, T >( q, t, self, dense, eps, pairs, cap, ps, dense_stack_limit, &it, &grid, &dense );
+  trav_item_t< K, T >( q, t, self, dense, alone, eps, pairs, cap, ps, dense_stack_limit, &it, &grid, &dense );
   // both objects' element slabs stored (dense contact): the walk that only reads them; else the one that computes the
   // slabs it tests from the vertices (unrolled when both objects have the same vertex count)
   if ( dense ) return walk_kernels< K, T, 0, true >::launch( it, grid, s );
@@ -1130,16 +1162,16 @@ cudaError_t launch_gather_words(const int *const *src, int n, int *dst, cudaStre
 }
 
 cudaError_t launch_traverse(int K, bool fp32, tree_view q, tree_view t, bool self, bool dense, double eps, uint2 *pairs,
-                            uint64_t cap, pair_scalars *ps, cudaStream_t s, int dense_stack_limit)
+                            uint64_t cap, pair_scalars *ps, cudaStream_t s, int dense_stack_limit, bool alone)
 {
   switch ( K )
   {
-    case 6: return fp32 ? launch_trav_t< 6, float >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit )
-                        : launch_trav_t< 6, double >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit );
-    case 18: return fp32 ? launch_trav_t< 18, float >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit )
-                         : launch_trav_t< 18, double >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit );
-    case 26: return fp32 ? launch_trav_t< 26, float >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit )
-                         : launch_trav_t< 26, double >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit );
+    case 6: return fp32 ? launch_trav_t< 6, float >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit, alone )
+                        : launch_trav_t< 6, double >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit, alone );
+    case 18: return fp32 ? launch_trav_t< 18, float >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit, alone )
+                         : launch_trav_t< 18, double >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit, alone );
+    case 26: return fp32 ? launch_trav_t< 26, float >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit, alone )
+                         : launch_trav_t< 26, double >( q, t, self, dense, eps, pairs, cap, ps, s, dense_stack_limit, alone );
     default: return cudaErrorInvalidValue;
   }
 }
@@ -1175,8 +1207,8 @@ void traverse_item(int K, bool fp32, tree_view q, tree_view t, bool self, bool d
                    bool *dense_out)
 {
   // the item's fields do not depend on K or the slab type; only the grid depends on K through nothing either
-  if ( fp32 ) trav_item_t< 18, float >( q, t, self, dense, eps, pairs, cap, ps, dense_stack_limit, item, blocks, dense_out );
-  else trav_item_t< 18, double >( q, t, self, dense, eps, pairs, cap, ps, dense_stack_limit, item, blocks, dense_out );
+  if ( fp32 ) trav_item_t< 18, float >( q, t, self, dense, false, eps, pairs, cap, ps, dense_stack_limit, item, blocks, dense_out );
+  else trav_item_t< 18, double >( q, t, self, dense, false, eps, pairs, cap, ps, dense_stack_limit, item, blocks, dense_out );
   (void)K;
 }
 
