@@ -389,6 +389,7 @@ struct trav_item
   pair_scalars *ps;
   int dense_stack;
   uint32_t width;  // queries per packet of the walk over stored slabs
+  uint32_t chunk;  // packets per chunk of the walk that computes slabs
   const obj_scalars *qsc;
 };
 
