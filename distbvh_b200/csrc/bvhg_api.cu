@@ -72,7 +72,7 @@ struct object
   // test from the vertices instead of storing all of them.
   bool store_slabs = false;
   bool stored = false;  // the last build stored them
-  // The batched dense walk reached its stack bound on this object's tree: its traversals use the single-node walk
+  // The walk over stored slabs reached its stack bound on this object's tree: its traversals compute their slabs
   // until the element count changes.
   bool dense_ok = true;
   // Patches (bvhg_cluster): valid until the next set_elements or rebuild.
@@ -204,7 +204,7 @@ struct bvhg_ctx
   bool own_stream = false;
   uint32_t spin_limit = kDefaultSpinLimit;
   int stall_sort = 0;  // test hook: radix look-back polls a status row nobody publishes
-  int dense_stack = 0;  // test hook: lower stack bound of the batched dense walk (0 = its own)
+  int dense_stack = 0;  // test hook: lower stack bound of the walk over stored slabs (0 = its own)
   std::vector< std::unique_ptr< object > > objs;
   cudaEvent_t fork_evt = nullptr;
   std::string err;
@@ -616,7 +616,7 @@ bvhg_status find_pairs(bvhg_ctx *ctx, object &a, object &b, bool self, const uin
     if ( st != BVHG_OK ) return st;
     if ( ctx->host_ps->error == kErrOverflowStack && dense && a.stored && b.stored )
     {
-      // the batched dense walk reached its stack bound: search again with the single-node walk
+      // the walk over stored slabs reached its stack bound: search again with computed slabs
       a.dense_ok = false;
       b.dense_ok = false;
       continue;
@@ -1254,7 +1254,7 @@ bvhg_status run_batch(bvhg_ctx *ctx, const batch_args &x, uint64_t *counts)
       const pair_scalars &h = B.host_ps[sc];
       if ( h.error == kErrOverflowStack && ctx->objs[x.a[sc]]->dense_ok && ctx->objs[x.b[sc]]->dense_ok )
       {
-        // the batched dense walk reached its stack bound: this scene's objects take the single-node walk and the
+        // the walk over stored slabs reached its stack bound: this scene's objects compute their slabs and the
         // batch runs again (a new layout: the graph is captured again)
         ctx->objs[x.a[sc]]->dense_ok = false;
         ctx->objs[x.b[sc]]->dense_ok = false;

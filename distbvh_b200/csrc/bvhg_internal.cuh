@@ -431,8 +431,8 @@ struct gid_args
 cudaError_t launch_gid_pairs_dev_batch(const batch_launch &b, cudaStream_t s);
 
 // Queries every leaf of q against tree t; writes (q element, t element) local index pairs. dense (both objects'
-// element slabs stored): the walk that pops nodes in batches and tests leaves in batches; its deeper stack bound can
-// be reached (ps->error = kErrOverflowStack), and the single-node walk (dense = false) then always completes.
+// element slabs stored): the walk that only reads them; its stack bound can, under a test hook,
+// be reached (ps->error = kErrOverflowStack), and the walk that computes slabs (dense = false) then always completes.
 // dense_stack_limit > 0 lowers that bound (test hook); 0 keeps it. alone: nothing else runs beside the search, so that a
 // small q may take packets of fewer queries (one scene of a batch shares the device).
 cudaError_t launch_traverse(int K, bool fp32, tree_view q, tree_view t, bool self, bool dense, double eps, uint2 *pairs,

@@ -237,7 +237,7 @@ BVHG_API bvhg_status bvhg_test_stall_sort(bvhg_ctx *ctx, int32_t enable);
  * `lanes` streams; else the fused form with that many groups of objects on `lanes` streams, lanes 1..64). */
 BVHG_API bvhg_status bvhg_test_batch_form(bvhg_ctx *ctx, uint32_t groups, uint32_t lanes);
 /* Test hook: lowers the stack bound of the dense-contact walk to `limit` entries (0 restores it), so that it is
- * reached and the library's fallback to the single-node walk runs (the pair set stays exact). */
+ * reached and the library's fallback to the walk that computes slabs runs (the pair set stays exact). */
 BVHG_API bvhg_status bvhg_test_dense_stack(bvhg_ctx *ctx, int32_t limit);
 
 /* Stable sort of n device-resident 64-bit keys (Morton keys or any others): keys_out[r] is the r-th smallest key,
