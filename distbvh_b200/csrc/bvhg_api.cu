@@ -1978,7 +1978,12 @@ bvhg_status bvhg_validate_tree(bvhg_ctx *ctx, int32_t obj, uint32_t *depth_out)
   for ( uint64_t r = 0; r < n; ++r )
   {
     if ( perm[r] >= n ) return fail( ctx, BVHG_ERR_STATE, "permutation entry out of range" );
-    for ( int k = 0; k < 2 * D; ++k ) eb[r * D * 2 + k] = lb[static_cast< size_t >( perm[r] ) * D * 2 + k];
+    for ( int k = 0; k < 2 * D; ++k )
+    {
+      // a slab that is not a number is the empty one, as the slab kernel unites it (no_slab)
+      const double v = lb[static_cast< size_t >( perm[r] ) * D * 2 + k];
+      eb[r * D * 2 + k] = v == v ? v : ( k & 1 ? -INFINITY : INFINITY );
+    }
   }
   // union of ranks [lo, hi) into out (2 D values)
   auto unite = [&](uint64_t lo, uint64_t hi, std::vector< double > &out) {

@@ -450,30 +450,7 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
     if ( valid ) slabs_to_row< K, T, VT >( x.qverts, x.qV, qe, x.eps, x.eps_hi, sm.q[lane] );
   }
   sm.qe[lane] = qe;
-  if ( width == 32u )
-  {
-    if ( lane < K ) sm.g[lane] = __ldg( wb + lane );
-    __syncwarp();
-  } else {
-    __syncwarp();
-    if ( lane < D )
-    {
-      // the union of the packet's rows (lanes past them hold its first one)
-      T lo, hi;
-      shared_pair( &sm.q[0][2 * lane], lo, hi );
-      const uint32_t rows = min( width, x.nq - i0 );
-      for ( uint32_t j = 1; j < rows; ++j )
-      {
-        T l, h;
-        shared_pair( &sm.q[j][2 * lane], l, h );
-        lo = l < lo ? l : lo;
-        hi = hi < h ? h : hi;
-      }
-      sm.g[2 * lane] = lo;
-      sm.g[2 * lane + 1] = hi;
-    }
-    __syncwarp();
-  }
+  __syncwarp();
   bool in_root = valid;
 #pragma unroll
   for ( int a = 0; a < D; ++a )
@@ -487,6 +464,26 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
   w.lane = lane;
   w.in = __ballot_sync( 0xffffffffu, in_root );
   if ( !w.in ) return;
+  // 3. The packet's union box: the group's, or that of the narrow packet's queries which overlap the root (their slabs
+  // are numbers; a NaN of another query must not reach the box).
+  if ( width == 32u )
+  {
+    if ( lane < K ) sm.g[lane] = __ldg( wb + lane );
+  } else if ( lane < D ) {
+    unsigned m = w.in;
+    T lo, hi;
+    shared_pair( &sm.q[__ffs( m ) - 1][2 * lane], lo, hi );
+    while ( m &= m - 1u )
+    {
+      T l, h;
+      shared_pair( &sm.q[__ffs( m ) - 1][2 * lane], l, h );
+      lo = l < lo ? l : lo;
+      hi = hi < h ? h : hi;
+    }
+    sm.g[2 * lane] = lo;
+    sm.g[2 * lane + 1] = hi;
+  }
+  __syncwarp();
   const int root = x.tsc->root;
   const unsigned lt = ( 1u << lane ) - 1u;
   const int limit = STORED ? x.stack_limit : kWalkStack;

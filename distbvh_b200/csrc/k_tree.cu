@@ -232,7 +232,11 @@ __device__ void slabs_body(const slabs_args &args, uint32_t bid, uint32_t nblk)
       T lo[D], hi[D];
       leaf_slabs< K, T, VT >( verts, Vrt, e, eps, eps_hi, lo, hi );
 #pragma unroll
-      for ( int a = 0; a < D; ++a ) io::store2( row + 2 * a, lo[a], hi[a] );
+      for ( int a = 0; a < D; ++a )
+      {
+        no_slab( lo[a], hi[a] );
+        io::store2( row + 2 * a, lo[a], hi[a] );
+      }
     }
     e = en;
     en = element( g + 2 * stride );

@@ -400,6 +400,18 @@ __device__ __forceinline__ void group_slabs64(const double *p, double eps, doubl
   }
 }
 
+// A slab that is not a number overlaps nothing. As (+inf, -inf) it still overlaps nothing, and the union of a box with
+// it is the box, where std_min and std_max would keep the NaN of a box's first element and lose the others.
+__device__ __forceinline__ void no_slab(double &l, double &h)
+{
+  if ( l != l || h != h )
+  {
+    l = __longlong_as_double( 0x7ff0000000000000LL );
+    h = -l;
+  }
+}
+__device__ __forceinline__ void no_slab(float &, float &) {}  // fminf and fmaxf already skip a NaN
+
 // Slabs of an element from its V vertices in registers, (min, max) per slab into a row aligned to such a pair.
 template< int K, typename T, int V >
 __device__ __forceinline__ void vertex_slabs(const double *p, double eps, float eps_hi, T *row)
@@ -407,7 +419,8 @@ __device__ __forceinline__ void vertex_slabs(const double *p, double eps, float 
   constexpr int D = K / 2;
   if constexpr ( sizeof( T ) == 8 )
   {
-    // Non-finite coordinates (which only a refit can meet) take the reference's operation order.
+    // Non-finite coordinates (which only a refit can meet) take the reference's operation order; a slab that is no
+    // number becomes the empty one (no_slab).
     unsigned most = 0;
 #pragma unroll
     for ( int k = 0; k < V * 3; ++k ) most = max( most, static_cast< unsigned >( __double2hiint( p[k] ) ) & 0x7ff00000u );
@@ -423,6 +436,7 @@ __device__ __forceinline__ void vertex_slabs(const double *p, double eps, float 
     {
       double l, h;
       slab64< K >( p, V, a, eps, l, h );
+      no_slab( l, h );
       *reinterpret_cast< double2 * >( row + 2 * a ) = make_double2( l, h );
     }
   } else {

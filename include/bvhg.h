@@ -128,6 +128,8 @@ BVHG_API bvhg_status bvhg_object_destroy(bvhg_ctx *ctx, int32_t obj);
 BVHG_API bvhg_status bvhg_set_elements(bvhg_ctx *ctx, int32_t obj, const double *xyz, uint32_t verts_per_elem,
                               const uint64_t *gid, uint64_t n, int32_t mem);
 
+/* A rebuild of elements with a non-finite coordinate fails (BVHG_ERR_ARG, reported by the next call that waits). A refit
+ * does not look for them: an element with a slab that is not a number overlaps nothing, the others keep their pairs. */
 BVHG_API bvhg_status bvhg_build(bvhg_ctx *ctx, int32_t obj, int32_t mode);
 
 /* Inter-object pairs: pairs[2p] = gid in obj_a, pairs[2p + 1] = gid in obj_b. mem = bvhg_mem of pairs.
