@@ -1615,7 +1615,8 @@ bvhg_status bvhg_sort_and_sweep(bvhg_ctx *ctx, int32_t obj_a, int32_t obj_b, int
   object &a = *ctx->objs[obj_a];
   object &b = *ctx->objs[obj_b];
   if ( !a.built || !b.built ) return fail( ctx, BVHG_ERR_STATE, "sort-and-sweep before build" );
-  // the global range and the axis come from the objects' bounds and centroids, which only a rebuild computes
+  // the axis comes from the objects' centroids, which only a rebuild computes (and only a rebuild refuses non-finite
+  // coordinates)
   if ( !a.fresh || !b.fresh ) return fail( ctx, BVHG_ERR_STATE, "sort-and-sweep needs a rebuild (not a refit) since set_elements" );
   cudaSetDevice( ctx->cfg.device );
   join_object( ctx, a );
@@ -1633,7 +1634,7 @@ bvhg_status bvhg_sort_and_sweep(bvhg_ctx *ctx, int32_t obj_a, int32_t obj_b, int
   BVHG_CUDA( ctx, ctx->sw_vals.reserve( 2 * nb4 * 4 ) );
   BVHG_CUDA( ctx, ctx->sw_srows.reserve( nb * K * 8 ) );
   BVHG_CUDA( ctx, ctx->sw_start.reserve( sweep_start_bytes() ) );
-  BVHG_CUDA( ctx, ctx->sw_hist.reserve( 2 * 256 * 4 ) );
+  BVHG_CUDA( ctx, ctx->sw_hist.reserve( sweep_hist_words() * 4 ) );
   BVHG_CUDA( ctx, ctx->sw_status.reserve( status_words * 4 ) );
   BVHG_CUDA( ctx, ctx->sw_sc.reserve( sizeof( obj_scalars ) ) );
   BVHG_CUDA( ctx, ctx->sw_params.reserve( sweep_params_bytes() ) );
@@ -1663,8 +1664,6 @@ bvhg_status bvhg_sort_and_sweep(bvhg_ctx *ctx, int32_t obj_a, int32_t obj_b, int
   x.bcx = b.cx.as< double >();
   x.bcy = b.cy.as< double >();
   x.bcz = b.cz.as< double >();
-  x.asc = a.sc();
-  x.bsc = b.sc();
   x.partial = ctx->sw_partial.as< double >();
   x.params = ctx->sw_params.p;
   x.keys = k0;
@@ -1682,7 +1681,7 @@ bvhg_status bvhg_sort_and_sweep(bvhg_ctx *ctx, int32_t obj_a, int32_t obj_b, int
     x.pairs = ctx->pairs.as< uint2 >();
     x.cap = ctx->pair_cap;
     BVHG_CUDA( ctx, cudaMemsetAsync( ssc, 0, sizeof( obj_scalars ), s ) );
-    BVHG_CUDA( ctx, cudaMemsetAsync( x.hist, 0, 2 * 256 * 4, s ) );
+    BVHG_CUDA( ctx, cudaMemsetAsync( x.hist, 0, sweep_hist_words() * 4, s ) );
     BVHG_CUDA( ctx, cudaMemsetAsync( ctx->sw_status.p, 0, status_words * 4, s ) );
     BVHG_CUDA( ctx, cudaMemsetAsync( ps, 0, sizeof( pair_scalars ), s ) );
     BVHG_CUDA( ctx, launch_sweep_setup( x, axis ) );

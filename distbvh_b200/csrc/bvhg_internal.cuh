@@ -269,11 +269,10 @@ struct sweep_launch
   uint64_t na, nb;
   double eps;
   const double *acx, *acy, *acz, *bcx, *bcy, *bcz;  // centroids (axis choice)
-  const obj_scalars *asc, *bsc;                     // K1 bounds of both objects (global range)
   double *partial;                                  // sweep_partial_bytes()
   void *params;                                     // sweep_params_bytes()
   uint64_t *keys;                                   // nb: B's (strip, bin) keys, original order
-  uint32_t *hist;                                   // 2 * 256: byte histograms of the keys
+  uint32_t *hist;                                   // sweep_hist_words(), zero: byte histograms of the keys, a counter
   const uint64_t *skeys;                            // sorted keys
   const uint32_t *svals;                            // B's element indices in key order
   uint32_t *start;                                  // sweep_start_bytes(): first position of every cell
@@ -288,8 +287,9 @@ struct sweep_launch
 size_t sweep_params_bytes();
 size_t sweep_partial_bytes();
 size_t sweep_start_bytes();
+constexpr size_t sweep_hist_words() { return 2 * 256 + 1; }
 int sweep_axis_read(const void *params_host_copy);
-// The axis (axis < 0: the one of largest centroid variance) and its scale factor, from the objects' bounds.
+// The axis (axis < 0: the one of largest centroid variance) and the borders of the strips, quantiles of B's slab minima.
 cudaError_t launch_sweep_setup(const sweep_launch &x, int axis);
 // B's keys, byte histograms and largest widths.
 cudaError_t launch_sweep_keys(const sweep_launch &x);

@@ -2,24 +2,31 @@
 //
 // Follows sort_and_sweep_local (src/bvh/narrowphase/kokkos.hpp:164-248) with the two objects as the two patches,
 // and max_variant_axis (kokkos.hpp:125-160) for the sweep axis when the caller gives none:
-// - the global range on the axis is the union of both objects' slab extents there (the K1 bounds of each object:
-//   min of the cardinal slab minima, max of the maxima);
-// - the reference scales B's slab minima on the axis to u32 keys, sorts them stably, and lets every element of A
-//   sweep B in key order: it skips the B elements that end before its minimum, stops at the first that begins after
-//   its maximum, and emits those that overlap it strictly on every slab. The emitted set is the exact pair set S(A, B)
-//   for any axis.
+// the reference scales B's slab minima on the axis to u32 keys over the union of both objects' extents, sorts them
+// stably, and lets every element of A sweep B in key order: it skips the B elements that end before its minimum, stops
+// at the first that begins after its maximum, and emits those that overlap it strictly on every slab. The emitted set is
+// the exact pair set S(A, B) for any axis.
 // The emitted set is that of the strict all-slab overlap, so the order in which candidates are met is free. A one
 // dimensional sweep of three dimensional elements meets thousands of them per element (two soups of 262,144 triangles:
 // 4,000 B elements in every window). Here the sweep axis is cut into 256 strips and every strip is swept on a
-// second axis (of the other two the one of larger extent), cut into 256 bins: B's key is (strip of its slab minimum,
-// bin of its second slab minimum), 16 bits, two radix passes, and start[] holds the first sorted position of every
-// (strip, bin) cell. An element of A then sweeps, in each strip of [its minimum - W, its maximum], the positions of
-// the bins of [its second minimum - W2, its second maximum], where W and W2 are the largest widths of a B element on
-// the two axes. Every overlapping B element lies there: b.min < a.max, and b.min >= b.max - W > a.min - W, with W
-// rounded up, a.min - W rounded down and the strip a monotone function of the value. The candidates are tested on the
-// third axis first, whose slabs lie contiguously in sorted order, then on the other slabs. The call on those two soups
-// takes 0.40 ms instead of 4.46 ms.
-// A degenerate axis (global_max == global_min) puts every element into strip or bin 0.
+// second axis (of the other two the one on which B's minima spread further), cut into 256 bins: B's key is (strip of its
+// slab minimum, bin of its second slab minimum), 16 bits, two radix passes, and start[] holds the first sorted position
+// of every (strip, bin) cell. An element of A then sweeps, in each strip of [its minimum - W, its maximum], the
+// positions of the bins of [its second minimum - W2, its second maximum], where W and W2 are the largest widths of a B
+// element on the two axes. Every overlapping B element lies there: b.min < a.max, and b.min >= b.max - W > a.min - W,
+// with W rounded up, a.min - W rounded down and the strip a monotone function of the value. The candidates are tested on
+// the third axis first, whose slabs lie contiguously in sorted order, then on the other slabs.
+// The borders of the strips (and bins) follow B's elements wherever they lie: 32 quantiles of B's slab minima, from a
+// sample of 1,024, and 8 even steps to the next one. A strip holds about nb / 256 elements, and a sweep meets at most two
+// partial strips beyond the elements that a one dimensional window holds. (Even steps over the objects' extents took the
+// same time for a uniform soup, but with one element 1,000 extents away nearly all of B lay in one cell and every element
+// of A met all of it.) Two soups of 262,144 triangles, us per call, with one dimensional windows of 32-bit keys, with even
+// steps, and now:
+//   uniform                                        3,850     300     300
+//   one element of B (or of A) 1,000 extents away  3,960 152,000     300
+//   two clusters 30 extents apart                  2,190   1,730     267
+//   normal deviates cubed                         11,900  54,000  11,200 (its dense middle holds most of the pairs)
+//   A 100 times as wide and as coarse              6,150   6,300   2,600
 #include "bvhg_internal.cuh"
 #include "kdop_math.cuh"
 
@@ -32,22 +39,52 @@ constexpr int kAxisBlocks = 512;  // partial sums of the axis choice (a fixed gr
 
 constexpr int kStrips = 256;  // strips of the sweep axis and bins of the second axis: one key byte each
 constexpr int kCells = kStrips * kStrips;
+constexpr int kKnots = 32;            // quantiles per axis
+constexpr int kSteps = kStrips / kKnots;  // strips between two of them
+constexpr int kSample = 1024;         // minima sampled per axis for them
 
 struct sweep_params
 {
   int axis;  // the sweep axis (read back by the host)
-  int axis2, axis3;
   int pad;
-  double gmin[2], fac[2];         // range minimum and scale factor of the sweep axis and the second axis
-  unsigned long long wmax_enc[2]; // order-preserving encodings of W and W2
+  unsigned long long wmax_enc[2];  // order-preserving encodings of W and W2
+  double knot[3][kKnots + 1];      // per axis: quantiles of B's slab minima, ascending
+  int axis2, axis3;
+  double2 cut[2][kKnots];          // of the sweep axis and the second axis: (knot, strips per unit after it)
 };
 
-// Strip (or bin) of a value: monotone in v; NaN gives 0.
-__device__ __forceinline__ uint32_t strip_of(double v, const sweep_params &p, int which)
+// The second axis: of the other two the one on which the middle three quarters of B's minima spread further.
+__device__ __forceinline__ int second_axis(const sweep_params *p, int axis)
 {
-  const double t = __dmul_rn( __dsub_rn( v, p.gmin[which] ), p.fac[which] );
-  if ( !( t >= 0.0 ) ) return 0u;
-  return t >= static_cast< double >( kStrips - 1 ) ? kStrips - 1 : static_cast< uint32_t >( t );
+  const int u = axis == 0 ? 1 : 0, v = axis == 2 ? 1 : 2;
+  constexpr int q0 = kKnots / 8, q1 = kKnots - q0;
+  return p->knot[v][q1] - p->knot[v][q0] > p->knot[u][q1] - p->knot[u][q0] ? v : u;
+}
+
+// Strip (or bin) of a value: monotone in v (NaN gives 0). Between two knots the strips are even steps; equal knots, whose
+// strips per unit are infinite, and knots further apart than a double tells still give a step in [0, kSteps).
+__device__ __forceinline__ uint32_t strip_between(double v, uint32_t q, double knot, double per_unit)
+{
+  const double t = __dmul_rn( __dsub_rn( v, knot ), per_unit );
+  return q * kSteps + ( t > 0.0 ? ( t < static_cast< double >( kSteps ) ? static_cast< uint32_t >( t ) : kSteps - 1u ) : 0u );
+}
+__device__ __forceinline__ uint32_t strip_of(double v, const double *knot, const double *per_unit)
+{
+  uint32_t q = 0;
+#pragma unroll
+  for ( uint32_t step = kKnots / 2; step > 0; step >>= 1 )
+    if ( knot[q + step] <= v ) q += step;
+  return strip_between( v, q, knot[q], per_unit[q] );
+}
+// The same by a whole warp whose lane q holds knot q and the strips per unit after it.
+__device__ __forceinline__ uint32_t strip_of(double v, double knot, double per_unit)
+{
+  static_assert( kKnots == 32, "one knot per lane" );
+  uint32_t q = 0;
+#pragma unroll
+  for ( uint32_t step = kKnots / 2; step > 0; step >>= 1 )
+    if ( __shfl_sync( 0xffffffffu, knot, q + step ) <= v ) q += step;
+  return strip_between( v, q, __shfl_sync( 0xffffffffu, knot, q ), __shfl_sync( 0xffffffffu, per_unit, q ) );
 }
 
 // The minimum and maximum of one coordinate over an element's vertices, with the inflation: the cardinal slab.
@@ -64,108 +101,165 @@ __device__ __forceinline__ void cardinal_slab(const double *__restrict__ src, in
   hi = __dadd_rn( mx, eps );
 }
 
-// Partial sums of the centroids and their squares over A then B (block b: a grid-stride range), fixed order.
-__global__ void __launch_bounds__( kSweepThreads ) k_axis_partial(const double *__restrict__ ax,
-                                                                  const double *__restrict__ ay,
-                                                                  const double *__restrict__ az, uint64_t na,
-                                                                  const double *__restrict__ bx,
-                                                                  const double *__restrict__ by,
-                                                                  const double *__restrict__ bz, uint64_t nb,
-                                                                  double *__restrict__ partial)
-{
-  __shared__ double s_red[6][kSweepThreads];
-  double s[6] = { 0, 0, 0, 0, 0, 0 };
-  const uint64_t n = na + nb;
-  for ( uint64_t i = static_cast< uint64_t >( blockIdx.x ) * kSweepThreads + threadIdx.x; i < n;
-        i += static_cast< uint64_t >( gridDim.x ) * kSweepThreads )
-  {
-    const double x = i < na ? ax[i] : bx[i - na];
-    const double y = i < na ? ay[i] : by[i - na];
-    const double z = i < na ? az[i] : bz[i - na];
-    s[0] = __dadd_rn( s[0], x );
-    s[1] = __dadd_rn( s[1], y );
-    s[2] = __dadd_rn( s[2], z );
-    s[3] = __dadd_rn( s[3], __dmul_rn( x, x ) );
-    s[4] = __dadd_rn( s[4], __dmul_rn( y, y ) );
-    s[5] = __dadd_rn( s[5], __dmul_rn( z, z ) );
-  }
-  for ( int k = 0; k < 6; ++k ) s_red[k][threadIdx.x] = s[k];
-  __syncthreads();
-  for ( int h = kSweepThreads / 2; h > 0; h >>= 1 )
-  {
-    if ( static_cast< int >( threadIdx.x ) < h )
-      for ( int k = 0; k < 6; ++k ) s_red[k][threadIdx.x] = __dadd_rn( s_red[k][threadIdx.x], s_red[k][threadIdx.x + h] );
-    __syncthreads();
-  }
-  if ( threadIdx.x < 6 ) partial[blockIdx.x * 6 + threadIdx.x] = s_red[threadIdx.x][0];
-}
+// Blocks [0, 3 per): the knots of the three axes, per blocks each. The sample takes one element of each of cnt equal
+// ranges of B (step elements each), its place in the range from a hash (an even stride would meet the same row of a
+// lattice again and again). The sample is not sorted: every block reads all of its axis and ranks 32 of its minima, 8
+// lanes per minimum and an eighth of the sample each, and the minima whose ranks are the quantiles write themselves. (A
+// bitonic network over 2,048 minima in one block per axis made a call 28 us longer.)
+// The other blocks (none when the caller gives the axis): partial sums of the centroids and their squares over A then B,
+// a grid-stride range each, fixed order, and the axis of largest centroid variance from them.
+constexpr int kRankLanes = 8;
 
-// The axis (given, or of largest centroid variance), the second axis, the global ranges on both and the scale
-// factors. The partial sums are added in block order (one lane per sum, from shared memory: a single thread reading
-// them from global memory took 135 us), so the axis does not depend on the run.
-__global__ void __launch_bounds__( 256 ) k_sweep_setup(const double *__restrict__ partial, int nblocks, uint64_t n,
-                                                       int axis_in, const obj_scalars *__restrict__ sa,
-                                                       const obj_scalars *__restrict__ sb, sweep_params *__restrict__ p)
+__device__ __forceinline__ void set_axis(sweep_params *p, int axis)
 {
-  __shared__ double s_part[kAxisBlocks * 6];
-  __shared__ double s_sum[6];
-  int axis = axis_in;
-  if ( axis < 0 )
-  {
-    for ( int k = threadIdx.x; k < nblocks * 6; k += 256 ) s_part[k] = partial[k];
-    __syncthreads();
-    if ( threadIdx.x < 6 )
-    {
-      double s = 0;
-      for ( int b = 0; b < nblocks; ++b ) s = __dadd_rn( s, s_part[b * 6 + threadIdx.x] );
-      s_sum[threadIdx.x] = s;
-    }
-    __syncthreads();
-  }
-  if ( threadIdx.x != 0 ) return;
-  if ( axis < 0 )
-  {
-    double var[3];
-    for ( int k = 0; k < 3; ++k )
-      var[k] = __dsub_rn( s_sum[3 + k], __ddiv_rn( __dmul_rn( s_sum[k], s_sum[k] ), static_cast< double >( n ) ) );
-    axis = 0;
-    if ( var[1] > var[0] ) axis = 1;
-    if ( var[2] > var[axis] ) axis = 2;
-  }
-  double gmin[3], ext[3];
-  for ( int k = 0; k < 3; ++k )
-  {
-    const double amin = ord_decode( sa->bounds_enc[k] ), amax = ord_decode( sa->bounds_enc[3 + k] );
-    const double bmin = ord_decode( sb->bounds_enc[k] ), bmax = ord_decode( sb->bounds_enc[3 + k] );
-    gmin[k] = bmin < amin ? bmin : amin;
-    ext[k] = __dsub_rn( amax < bmax ? bmax : amax, gmin[k] );
-  }
-  const int u = axis == 0 ? 1 : 0, v = axis == 2 ? 1 : 2;  // the other two axes
-  const int axis2 = ext[v] > ext[u] ? v : u;
   p->axis = axis;
-  p->axis2 = axis2;
-  p->axis3 = 3 - axis - axis2;
-  p->gmin[0] = gmin[axis];
-  p->gmin[1] = gmin[axis2];
-  p->fac[0] = ext[axis] > 0.0 ? __ddiv_rn( static_cast< double >( kStrips ), ext[axis] ) : 0.0;
-  p->fac[1] = ext[axis2] > 0.0 ? __ddiv_rn( static_cast< double >( kStrips ), ext[axis2] ) : 0.0;
   p->wmax_enc[0] = p->wmax_enc[1] = ord_encode( 0.0 );
 }
 
-// B's keys, the histograms of their two bytes, and the largest widths on the two axes.
+__global__ void __launch_bounds__( kSweepThreads ) k_sweep_sample(sweep_launch x, int axis_in, int per, int cnt, double step)
+{
+  __shared__ alignas( 16 ) double s_val[6 * kSweepThreads];
+  static_assert( kSample <= 6 * kSweepThreads, "one array for both" );
+  const int t = threadIdx.x;
+  if ( static_cast< int >( blockIdx.x ) < 3 * per )
+  {
+    if ( axis_in >= 0 && blockIdx.x == 0 && t == 0 ) set_axis( static_cast< sweep_params * >( x.params ), axis_in );
+    const int k = blockIdx.x / per;
+    const int V = static_cast< int >( x.bV );
+    // a thread's samples together: one trip to memory per vertex
+    constexpr int PER = kSample / kSweepThreads;
+    const double *src[PER];
+    double mn[PER];
+#pragma unroll
+    for ( int q = 0; q < PER; ++q )
+    {
+      const int j = q * kSweepThreads + t;
+      src[q] = x.bverts + k;
+      if ( j < cnt )
+      {
+        uint32_t h = static_cast< uint32_t >( j ) + 1u;  // a 32-bit mixer of shifts and odd multipliers
+        h = ( h ^ ( h >> 16 ) ) * 0x7feb352du;
+        h = ( h ^ ( h >> 15 ) ) * 0x846ca68bu;
+        h ^= h >> 16;
+        const uint64_t e = static_cast< uint64_t >( __dmul_rn( j + h * 0x1p-32, step ) );
+        src[q] += min( e, x.nb - 1 ) * V * 3;
+      }
+      mn[q] = __ldg( src[q] );
+    }
+    for ( int v = 1; v < V; ++v )
+    {
+#pragma unroll
+      for ( int q = 0; q < PER; ++q ) mn[q] = std_min( mn[q], __ldg( src[q] + 3 * v ) );
+    }
+#pragma unroll
+    for ( int q = 0; q < PER; ++q ) s_val[q * kSweepThreads + t] = __dsub_rn( mn[q], x.eps );
+    __syncthreads();
+    // rank: the minima below it, and the equal ones before it
+    const int i = ( static_cast< int >( blockIdx.x ) % per ) * ( kSweepThreads / kRankLanes ) + t / kRankLanes;
+    const double mine = i < cnt ? s_val[i] : 0.0;
+    int rank = 0;
+#pragma unroll 8
+    for ( int j = t % kRankLanes; j < cnt; j += kRankLanes )
+    {
+      const double y = s_val[j];
+      rank += ( y < mine ) | ( ( y == mine ) & ( j < i ) );
+    }
+#pragma unroll
+    for ( int o = 1; o < kRankLanes; o <<= 1 ) rank += __shfl_xor_sync( 0xffffffffu, rank, o );
+    if ( i >= cnt || t % kRankLanes ) return;
+    // knot q is the minimum of rank q cnt / kKnots (q of one rank: consecutive, none or several), the last the largest
+    double *knot = static_cast< sweep_params * >( x.params )->knot[k];
+    for ( int q = ( rank * kKnots + cnt - 1 ) / cnt; q < kKnots && q * cnt / kKnots == rank; ++q ) knot[q] = mine;
+    if ( rank == cnt - 1 ) knot[kKnots] = mine;
+    return;
+  }
+  const uint64_t block = blockIdx.x - 3 * per, na = x.na, n = x.na + x.nb;
+  double s[6] = { 0, 0, 0, 0, 0, 0 };
+  for ( uint64_t i = block * kSweepThreads + t; i < n; i += static_cast< uint64_t >( kAxisBlocks ) * kSweepThreads )
+  {
+    const double c[3] = { __ldg( i < na ? x.acx + i : x.bcx + ( i - na ) ), __ldg( i < na ? x.acy + i : x.bcy + ( i - na ) ),
+                          __ldg( i < na ? x.acz + i : x.bcz + ( i - na ) ) };
+#pragma unroll
+    for ( int k = 0; k < 3; ++k )
+    {
+      s[k] = __dadd_rn( s[k], c[k] );
+      s[3 + k] = __dadd_rn( s[3 + k], __dmul_rn( c[k], c[k] ) );
+    }
+  }
+  for ( int k = 0; k < 6; ++k ) s_val[k * kSweepThreads + t] = s[k];
+  __syncthreads();
+  for ( int h = kSweepThreads / 2; h > 0; h >>= 1 )
+  {
+    if ( t < h )
+      for ( int k = 0; k < 6; ++k )
+        s_val[k * kSweepThreads + t] = __dadd_rn( s_val[k * kSweepThreads + t], s_val[k * kSweepThreads + t + h] );
+    __syncthreads();
+  }
+  if ( t < 6 )
+  {
+    x.partial[block * 6 + t] = s_val[t * kSweepThreads];
+    __threadfence();
+  }
+  __syncthreads();
+  // the last block to finish chooses the axis: the sums are added in block order (one lane per sum, from shared memory: a
+  // single thread reading them from global memory took 135 us), so it does not depend on the run
+  __shared__ bool s_last;
+  if ( t == 0 ) s_last = atomicAdd( x.hist + 2 * 256, 1u ) == kAxisBlocks - 1;
+  __syncthreads();
+  if ( !s_last ) return;
+  __threadfence();
+  __shared__ double s_part[kAxisBlocks * 6];
+  for ( int k = t; k < kAxisBlocks * 6; k += kSweepThreads ) s_part[k] = __ldcg( x.partial + k );
+  __syncthreads();
+  if ( t < 6 )
+  {
+    double sum = 0;
+#pragma unroll 4
+    for ( int b = 0; b < kAxisBlocks; ++b ) sum = __dadd_rn( sum, s_part[b * 6 + t] );
+    s_val[t] = sum;
+  }
+  __syncthreads();
+  if ( t != 0 ) return;
+  double var[3];
+  for ( int k = 0; k < 3; ++k )
+    var[k] = __dsub_rn( s_val[3 + k], __ddiv_rn( __dmul_rn( s_val[k], s_val[k] ), static_cast< double >( n ) ) );
+  int axis = 0;
+  if ( var[1] > var[0] ) axis = 1;
+  if ( var[2] > var[axis] ) axis = 2;
+  set_axis( static_cast< sweep_params * >( x.params ), axis );
+}
+
+// B's keys, the histograms of their two bytes, and the largest widths on the two axes. A grid of at most two blocks per
+// SM strides over the elements: every block adds up to 512 counts to the histograms, and those atomics were most of the
+// kernel with one block per 256 elements (262,144 elements 18.6 -> 12.1 us).
 __global__ void __launch_bounds__( kSweepThreads ) k_sweep_keys(const double *__restrict__ verts, int V, uint64_t n,
                                                                 double eps, const sweep_params *pp,
                                                                 uint64_t *__restrict__ keys, uint32_t *__restrict__ hist,
                                                                 sweep_params *pw)  // pp and pw: the same struct
 {
   __shared__ uint32_t s_hist[2 * 256];
+  __shared__ double s_knot[2][kKnots], s_per[2][kKnots];
   __shared__ double s_w[2][kSweepThreads / 32];
+  const int axis = pp->axis, axis2 = second_axis( pp, axis );
   for ( int k = threadIdx.x; k < 2 * 256; k += kSweepThreads ) s_hist[k] = 0;
-  const sweep_params p = *pp;
+  if ( threadIdx.x < 2 * kKnots )
+  {
+    const int c = threadIdx.x / kKnots, q = threadIdx.x % kKnots, a = c ? axis2 : axis;
+    const double from = pp->knot[a][q];
+    const double per_unit = __ddiv_rn( static_cast< double >( kSteps ), __dsub_rn( pp->knot[a][q + 1], from ) );
+    s_knot[c][q] = from;
+    s_per[c][q] = per_unit;
+    if ( blockIdx.x == 0 ) pw->cut[c][q] = make_double2( from, per_unit );  // for A's sweeps
+  }
+  if ( blockIdx.x == 0 && threadIdx.x == 0 )
+  {
+    pw->axis2 = axis2;
+    pw->axis3 = 3 - axis - axis2;
+  }
   __syncthreads();
-  const uint64_t i = static_cast< uint64_t >( blockIdx.x ) * kSweepThreads + threadIdx.x;
   double w[2] = { 0.0, 0.0 };
-  if ( i < n )
+  for ( uint64_t i = static_cast< uint64_t >( blockIdx.x ) * kSweepThreads + threadIdx.x; i < n;
+        i += static_cast< uint64_t >( gridDim.x ) * kSweepThreads )
   {
     const double *src = verts + i * V * 3;
     uint32_t key = 0;
@@ -173,9 +267,10 @@ __global__ void __launch_bounds__( kSweepThreads ) k_sweep_keys(const double *__
     for ( int c = 0; c < 2; ++c )
     {
       double lo, hi;
-      cardinal_slab( src, V, c ? p.axis2 : p.axis, eps, lo, hi );
-      key = ( key << 8 ) | strip_of( lo, p, c );
-      w[c] = __dsub_ru( hi, lo );
+      cardinal_slab( src, V, c ? axis2 : axis, eps, lo, hi );
+      key = ( key << 8 ) | strip_of( lo, s_knot[c], s_per[c] );
+      const double x = __dsub_ru( hi, lo );
+      w[c] = x > w[c] ? x : w[c];
     }
     keys[i] = key;
     atomicAdd( &s_hist[key & 255u], 1u );
@@ -187,7 +282,7 @@ __global__ void __launch_bounds__( kSweepThreads ) k_sweep_keys(const double *__
     for ( int o = 16; o > 0; o >>= 1 )
     {
       const double x = __shfl_xor_sync( 0xffffffffu, w[c], o );
-      w[c] = w[c] > x ? w[c] : ( x > w[c] ? x : ( w[c] == w[c] ? w[c] : x ) );
+      w[c] = x > w[c] ? x : w[c];
     }
     if ( ( threadIdx.x & 31 ) == 0 ) s_w[c][threadIdx.x >> 5] = w[c];
   }
@@ -250,8 +345,13 @@ constexpr int kPairThreads = 128;
 // A: a warp takes `per` (at most 32) consecutive elements of A in Morton order. Every lane forms the slabs and the
 // strip and bin ranges of one of them; then the warp sweeps them one after the other, 32 positions of a strip at a
 // time. All lanes forming the same element's slabs, one warp per element, cost as much as the sweep itself.
+// Resident blocks: the compiler's own choice of registers spilled in the sweep's loop or left fewer warps (triangles at
+// 18-DOP, 2 x 262,144: 338 us a call at 12 blocks, 290 at 8 to 9; hexahedra would get 3 blocks at 26-DOP).
 template< int K, int VT >
-__global__ void __launch_bounds__( kPairThreads ) k_sweep(const double *__restrict__ verts, uint32_t Vrt, uint64_t na,
+constexpr int kSweepMinBlocks = K == 6 ? 12 : ( VT == 8 ? ( K == 26 ? 4 : 5 ) : ( K == 26 ? 8 : 9 ) );
+
+template< int K, int VT >
+__global__ void __launch_bounds__( kPairThreads, kSweepMinBlocks< K, VT > ) k_sweep(const double *__restrict__ verts, uint32_t Vrt, uint64_t na,
                                                           uint32_t per, double eps, const sweep_params *__restrict__ pp,
                                                           const uint32_t *__restrict__ aperm,
                                                           const uint32_t *__restrict__ start,
@@ -263,13 +363,14 @@ __global__ void __launch_bounds__( kPairThreads ) k_sweep(const double *__restri
   constexpr int D = K / 2;
   __shared__ alignas( 16 ) double s_rows[kPairThreads / 32][32][K];
   if ( *reinterpret_cast< const volatile int * >( &ssc->error ) == kErrTimeout ) return;  // keys not sorted
-  const sweep_params p = *pp;
+  const int axis = pp->axis, axis2 = pp->axis2, axis3 = pp->axis3;
   const unsigned lane = threadIdx.x & 31u, lt = ( 1u << lane ) - 1u;
   double( *rows )[K] = s_rows[threadIdx.x >> 5];
-  const double2 *z = reinterpret_cast< const double2 * >( srows ) + static_cast< uint64_t >( p.axis3 ) * nb;
+  const double2 *z = reinterpret_cast< const double2 * >( srows ) + static_cast< uint64_t >( axis3 ) * nb;
   const uint64_t first = static_cast< uint64_t >( ( blockIdx.x * kPairThreads + threadIdx.x ) >> 5 ) * per;
   uint32_t i = 0, span = 0;  // span: first strip, last strip, first bin, last bin
-  if ( lane < per && first + lane < na )
+  const bool mine = lane < per && first + lane < na;
+  if ( mine )
   {
     i = __ldg( aperm + first + lane );
     double lo[D], hi[D];
@@ -280,13 +381,16 @@ __global__ void __launch_bounds__( kPairThreads ) k_sweep(const double *__restri
       rows[lane][2 * a] = lo[a];
       rows[lane][2 * a + 1] = hi[a];
     }
+  }
+  __syncwarp();  // the cuts are loaded here, not beside the vertices: their registers are free again
 #pragma unroll
-    for ( int c = 0; c < 2; ++c )
-    {
-      const int a = c ? p.axis2 : p.axis;
-      const double mn = a == 0 ? lo[0] : ( a == 1 ? lo[1] : lo[2] ), mx = a == 0 ? hi[0] : ( a == 1 ? hi[1] : hi[2] );
-      span |= ( strip_of( __dsub_rd( mn, ord_decode( p.wmax_enc[c] ) ), p, c ) | ( strip_of( mx, p, c ) << 8 ) ) << ( 16 * c );
-    }
+  for ( int c = 0; c < 2; ++c )
+  {
+    const double *slab = rows[lane] + 2 * ( c ? axis2 : axis );
+    const double mn = mine ? slab[0] : 0.0, mx = mine ? slab[1] : 0.0;
+    const double2 cut = __ldg( &pp->cut[c][lane] );
+    const uint32_t s0 = strip_of( __dsub_rd( mn, ord_decode( pp->wmax_enc[c] ) ), cut.x, cut.y );
+    span |= ( s0 | ( strip_of( mx, cut.x, cut.y ) << 8 ) ) << ( 16 * c );
   }
   __syncwarp();
   const uint32_t count = first < na ? static_cast< uint32_t >( min( static_cast< uint64_t >( per ), na - first ) ) : 0u;
@@ -295,7 +399,7 @@ __global__ void __launch_bounds__( kPairThreads ) k_sweep(const double *__restri
     const uint32_t ai = __shfl_sync( 0xffffffffu, i, u ), sp = __shfl_sync( 0xffffffffu, span, u );
     const uint32_t s0 = sp & 255u, s1 = ( sp >> 8 ) & 255u, y0 = ( sp >> 16 ) & 255u, y1 = sp >> 24;
     const double *row = rows[u];
-    const double zlo = row[2 * p.axis3], zhi = row[2 * p.axis3 + 1];
+    const double zlo = row[2 * axis3], zhi = row[2 * axis3 + 1];
     for ( uint32_t sb = s0; sb <= s1; sb += 32 )
     {
       uint32_t b = 0, e = 0;  // the positions of strip sb + lane
@@ -396,21 +500,20 @@ int sweep_axis_read(const void *params_host_copy) { return static_cast< const sw
 
 cudaError_t launch_sweep_setup(const sweep_launch &x, int axis)
 {
-  if ( axis < 0 )
-  {
-    k_axis_partial<<< kAxisBlocks, kSweepThreads, 0, x.s >>>( x.acx, x.acy, x.acz, x.na, x.bcx, x.bcy, x.bcz, x.nb,
-                                                             x.partial );
-    cudaError_t e = cudaGetLastError();
-    if ( e != cudaSuccess ) return e;
-  }
-  k_sweep_setup<<< 1, 256, 0, x.s >>>( x.partial, kAxisBlocks, x.na + x.nb, axis, x.asc, x.bsc,
-                                       static_cast< sweep_params * >( x.params ) );
+  // a quarter of the sample below 16,384 elements: the ranking of 256 ends before the axis beside it, that of 1,024 made a
+  // call on 2 x 1,000 triangles 110 us instead of 101; from there on the more even strips are worth it (2 x 40,000: 147
+  // instead of 149 us)
+  const uint64_t want = x.na < ( 1u << 14 ) || x.nb < ( 1u << 14 ) ? kSample / 4 : kSample;
+  const int cnt = static_cast< int >( x.nb < want ? x.nb : want ), per = ( cnt * kRankLanes + kSweepThreads - 1 ) / kSweepThreads;
+  k_sweep_sample<<< 3 * per + ( axis < 0 ? kAxisBlocks : 0 ), kSweepThreads, 0, x.s >>>( x, axis, per, cnt,
+                                                                                       static_cast< double >( x.nb ) / cnt );
   return cudaGetLastError();
 }
 
 cudaError_t launch_sweep_keys(const sweep_launch &x)
 {
-  const unsigned grid = static_cast< unsigned >( ( x.nb + kSweepThreads - 1 ) / kSweepThreads );
+  const uint64_t blocks = ( x.nb + kSweepThreads - 1 ) / kSweepThreads, most = 2 * static_cast< uint64_t >( device_sm_count() );
+  const unsigned grid = static_cast< unsigned >( blocks < most ? blocks : most );
   k_sweep_keys<<< grid, kSweepThreads, 0, x.s >>>( x.bverts, static_cast< int >( x.bV ), x.nb, x.eps,
                                                    static_cast< const sweep_params * >( x.params ), x.keys, x.hist,
                                                    static_cast< sweep_params * >( x.params ) );
