@@ -141,11 +141,12 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
 //     slabs against the packet's union box. A leaf bucket that passes goes onto the bucket list, an internal node back
 //     onto the stack; children smaller than half the packet's box go onto the check list first.
 //   - Check: lane = query. The cardinal slabs of the listed boxes are staged in shared memory, eight boxes at a time,
-//     and every lane tests its query against them. A child that no query overlaps is dropped.
+//     and every lane tests its query against them. A child that no query overlaps is dropped, and a bucket is listed
+//     with the queries that overlap it.
 //   - Filter: lane = element of four listed buckets. The elements that overlap the packet's union box are gathered, 16
-//     at a time, as rows in shared memory.
-//   - Cardinal tests: lane = (query of two, gathered element), the element's cardinal slabs in registers, over the
-//     packet's queries. Survivors collect in a list in shared memory.
+//     at a time, as rows in shared memory, and with them the queries of their buckets.
+//   - Cardinal tests: lane = (query of two, gathered element), the element's cardinal slabs in registers, over those
+//     queries. Survivors collect in a list in shared memory.
 //   - Slab tests: lane = survivor (query, element), on the other slabs.
 // Everything larger than a query costs one lane-test per box or element instead of 32. On a tet lattice at 26-DOP a
 // packet meets 157 nodes, 49 buckets of 390 elements, 149 elements that overlap its box, 310 survivors and 133 pairs
@@ -160,8 +161,11 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
 // against every bucket and four queries by eight elements per round from shared memory (15.4 ms); the same with a
 // second round for the non-cardinal slabs by (survivor, slab) lanes (29 ms); rows read five slabs at a time (20 to 50
 // ms, depending on the resident warps).
-// A packet whose ranks straddle a jump of the Morton curve, or whose elements lie far apart, has a union box that says
-// little: the check of the small children keeps its walk on the nodes that one of its queries overlaps.
+// A packet whose ranks straddle a jump of the Morton curve, or whose elements lie far apart, or one of whose elements is
+// long, has a union box that says little: the check of the small children keeps its walk on the nodes that one of its
+// queries overlaps, and the buckets' queries keep the cardinal tests on those. (Testing all queries of the packet against
+// every gathered element: 300,000 triangles of which 100 span half the domain against 300,000 small ones 15.1 ms instead
+// of 8.6, one in 1,000 spanning 0.3 of it 2.8 instead of 1.6 ms, and the even tet lattices above 4-5% more of a step.)
 //
 // The element slabs come from the rows that the slab kernel stored (STORED: dense contact; slab-major per bucket, so
 // that the filter reads the pairs of one slab of eight elements as one piece) or are computed from the vertices: the
@@ -189,8 +193,9 @@ struct walk_smem
   alignas( 16 ) T rows[kCheckRows][6];  // cardinal slabs of the boxes being checked
   alignas( 16 ) T g[K];                 // the packet's union box
   alignas( 16 ) uint2 out[kPairBuf];    // pairs found and not yet written
-  int2 list[kCheckCap];                 // (2 * parent + side, child link) to check
+  int list[kCheckCap];                  // children to check: 2 * parent + side
   int leaf[kLeafCap];                   // buckets to filter
+  unsigned mask[kLeafCap];              // the queries that may overlap each of them
   int stack[kWalkStack];                // internal nodes to expand
   uint32_t qe[32];                      // query element indices
   uint32_t te[kGather], tr[kGather];    // element indices and ranks of the gathered elements
@@ -204,6 +209,7 @@ struct walk_state
   unsigned lane;
   unsigned in;    // queries that overlap the target's root box
   int ne = 0;     // gathered elements
+  unsigned any = 0;  // queries that may overlap one of them
   uint32_t ns = 0, nout = 0;
 };
 
@@ -297,7 +303,7 @@ __device__ __forceinline__ void test_gathered(const trav_args< T > &x, walk_smem
   // self-collision: only the queries of lower rank
   const uint32_t above = act ? ( x.self ? sm.tr[e] - w.i0 : 32u ) : 0u;
   constexpr int U = 2;
-  for ( unsigned m = w.in; m; )
+  for ( unsigned m = w.any; m; )
   {
     uint32_t q[U];
     bool ok[U];
@@ -357,6 +363,7 @@ __device__ __forceinline__ void test_gathered(const trav_args< T > &x, walk_smem
   }
   __syncwarp();
   w.ne = 0;
+  w.any = 0;
 }
 
 // The filter of the nleaf listed buckets.
@@ -413,6 +420,7 @@ __device__ __forceinline__ void filter_buckets(const trav_args< T > &x, walk_sme
         }
       }
       w.ne = min( kGather, w.ne + __popc( m ) );
+      w.any |= __reduce_or_sync( 0xffffffffu, put ? sm.mask[b] : 0u );
       m &= ~__ballot_sync( 0xffffffffu, put );
       if ( w.ne == kGather ) test_gathered( x, sm, w );
     }
@@ -491,6 +499,7 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
   bool full = false;  // the stack bound was reached (uniform over the warp)
   if ( lane == 0 )
   {
+    sm.mask[0] = w.in;
     if ( root < 0 ) sm.leaf[0] = ~root;
     else sm.stack[0] = root;
   }
@@ -548,9 +557,13 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
       if ( full ) break;
       if ( o )
       {
-        if ( small ) sm.list[nl + __popc( ml & lt )] = make_int2( 2 * node + side, c );
+        if ( small ) sm.list[nl + __popc( ml & lt )] = 2 * node + side;
         else if ( c >= 0 ) sm.stack[sp + __popc( mp & lt )] = c;
-        else sm.leaf[nleaf + __popc( mb & lt )] = ~c;
+        else
+        {
+          sm.leaf[nleaf + __popc( mb & lt )] = ~c;
+          sm.mask[nleaf + __popc( mb & lt )] = w.in;
+        }
       }
       nl += __popc( ml );
       sp += __popc( mp );
@@ -561,13 +574,15 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
     for ( int b0 = 0; b0 < nl && !full; b0 += kCheckRows )
     {
       const int nb = min( kCheckRows, nl - b0 );
+      int link = 0;  // of the child whose slab this lane copies
       {
         static_assert( kCheckRows * 3 <= 32, "one pair per lane" );
         const int k = static_cast< int >( lane ) / 3, a = static_cast< int >( lane ) - 3 * k;
         if ( k < nb )
         {
-          const int e = sm.list[b0 + k].x;
+          const int e = sm.list[b0 + k];
           copy_pair( &sm.rows[k][2 * a], x.nbox + static_cast< size_t >( e >> 1 ) * D * 4 + a * 4 + ( e & 1 ) * 2 );
+          link = __ldg( reinterpret_cast< const int * >( x.child ) + e );
         }
       }
       cp_async_wait_all();
@@ -587,11 +602,11 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
           alive &= o ? ~0u : ~( 1u << j );
         }
       }
-      alive = __reduce_or_sync( 0xffffffffu, alive );  // bit j: some query overlaps box j
       for ( int j = 0; j < nb; ++j )
       {
-        if ( !( ( alive >> j ) & 1u ) ) continue;
-        const int ch = sm.list[b0 + j].y;
+        const unsigned who = __ballot_sync( 0xffffffffu, ( alive >> j ) & 1u );  // the queries that overlap box j
+        if ( !who ) continue;
+        const int ch = __shfl_sync( 0xffffffffu, link, 3 * j );
         if ( ch < 0 )
         {
           if ( nleaf == kLeafCap )
@@ -600,7 +615,11 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
             filter_buckets< K, T, VT, STORED >( x, sm, w, nleaf );
             nleaf = 0;
           }
-          if ( lane == 0 ) sm.leaf[nleaf] = ~ch;
+          if ( lane == 0 )
+          {
+            sm.leaf[nleaf] = ~ch;
+            sm.mask[nleaf] = who;
+          }
           ++nleaf;
         } else if ( sp < limit ) {
           if ( lane == 0 ) sm.stack[sp] = ch;
