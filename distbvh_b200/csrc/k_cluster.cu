@@ -460,8 +460,10 @@ __global__ void k_group_scatter(const uint2 *__restrict__ pairs, uint64_t np, gr
 // src/bvh/snapshot.hpp:139-149). A warp takes consecutive groups of 32 positions of the patch order: its lanes gather
 // the elements' vertices together and write one row of slabs each; then lane c unites component c of the rows, keeps
 // the union while the groups stay in one patch, and updates the patch's order-preserving encoding when they leave it.
-// A group that spans patches is united lane by lane. (One thread per position with its own loads, a shuffle reduction
-// of every slab and an atomic per group of 32 took 38 us for 327,680 triangles at 26-DOP; this takes 27 us.)
+// Patches of fewer than 32 elements are united and written one after the other. (One thread per position with its own
+// loads, a shuffle reduction of every slab and an atomic per group of 32 took 38 us for 327,680 triangles at 26-DOP; this
+// takes 27 us. A call on 300,000 triangles in patches of five: 100 us so, 115 us when their lanes each wrote their own
+// slabs, 75 us now; elements of six vertices 170, 220 and 73 us.)
 constexpr int kPatchThreads = 64;
 
 template< int K, int VT >
@@ -497,7 +499,7 @@ __global__ void __launch_bounds__( kPatchThreads ) k_patch_kdops(const double *_
     const int rows = static_cast< int >( min( 32u, n - 32 * g ) );
     const bool valid = lane < rows;
     const uint32_t e = valid ? __ldg( order + r ) : 0u;
-    const uint32_t first = patch_of( bounds, patches, 32 * g ), last = patch_of( bounds, patches, 32 * g + rows - 1 );
+    const uint32_t p = patch_of( bounds, patches, valid ? r : n - 1 );
     if constexpr ( VT > 0 )
     {
       gather_vertices< VT >( verts, e, rows, s_v[warp], lane );
@@ -508,8 +510,21 @@ __global__ void __launch_bounds__( kPatchThreads ) k_patch_kdops(const double *_
 #pragma unroll
       for ( int a = 0; a < D; ++a ) slab64< K >( v, VT, a, eps, row[2 * a], row[2 * a + 1] );
     } else if ( valid ) {
+      // one vertex after the other on all slabs: every coordinate is read once (leaf_slabs reads it once per slab)
       double lo[D], hi[D];
-      leaf_slabs< K, double, VT >( verts, Vrt, e, eps, 0.f, lo, hi );
+      const double *src = verts + static_cast< size_t >( e ) * Vrt * 3;
+      for ( uint32_t v = 0; v < Vrt; ++v )
+      {
+        const double x[3] = { __ldg( src + 3 * v ), __ldg( src + 3 * v + 1 ), __ldg( src + 3 * v + 2 ) };
+#pragma unroll
+        for ( int a = 0; a < D; ++a )
+        {
+          double l, h;
+          slab64< K >( x, 1, a, eps, l, h );
+          lo[a] = v ? std_min( lo[a], l ) : l;
+          hi[a] = v ? std_max( hi[a], h ) : h;
+        }
+      }
 #pragma unroll
       for ( int a = 0; a < D; ++a )
       {
@@ -518,26 +533,23 @@ __global__ void __launch_bounds__( kPatchThreads ) k_patch_kdops(const double *_
       }
     }
     __syncwarp();
-    if ( first == last )
+    // the group's patches one after the other (mostly one)
+    for ( int j = 0; j < rows; )
     {
-      if ( first != held )
+      const uint32_t pj = __shfl_sync( 0xffffffffu, p, j );
+      const int j1 = min( rows, j + __popc( __ballot_sync( 0xffffffffu, p == pj ) ) );
+      if ( pj != held )
       {
         flush();
-        held = first;
+        held = pj;
       }
       if ( lane < K )
-        for ( int j = 0; j < rows; ++j )
+        for ( ; j < j1; ++j )
         {
           const unsigned long long x = ord_encode( s_row[warp][j * P + lane] );
           acc = upper ? ( x > acc ? x : acc ) : ( x < acc ? x : acc );
         }
-    } else if ( valid ) {
-      unsigned long long *p = enc + static_cast< size_t >( patch_of( bounds, patches, r ) ) * K;
-      for ( int a = 0; a < D; ++a )
-      {
-        atomicMin( p + 2 * a, ord_encode( row[2 * a] ) );
-        atomicMax( p + 2 * a + 1, ord_encode( row[2 * a + 1] ) );
-      }
+      j = j1;
     }
     __syncwarp();  // the rows and the vertices are refilled by the next group
   }
