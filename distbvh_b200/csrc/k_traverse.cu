@@ -15,7 +15,6 @@
 // Self-collision (self_collision_set, collision_query.hpp:331-368): the query of rank i only visits subtrees
 // holding ranks > i (internal node k splits its bucket range [l, r] into [l, k] and [k + 1, r]) and tests only
 // bucket elements of rank > i, so every unordered pair is found once and no element is paired with itself.
-#include <atomic>
 #include <cstddef>
 
 #include "bulk_copy.cuh"
@@ -777,12 +776,13 @@ void trav_item_t(tree_view q, tree_view t, bool self, bool dense, bool alone, do
   *dense_out = dense;
 }
 
-// The shared-memory opt-in of a walk's two launch forms, once per device.
+// A walk's two launch forms.
 template< int K, typename T, int VT, bool STORED >
 struct walk_kernels
 {
   static constexpr int MB = kWalkBlocks< K, T, STORED >;
   static constexpr int smem = kWalkSmem< K, T, STORED >;
+  static_assert( smem <= 48 * 1024, "more shared memory per block needs the opt-in" );
   static constexpr auto single()
   {
     if constexpr ( STORED ) return &k_single< trav_item, stored_body< K, T >, kTravThreads, MB >;
@@ -793,31 +793,13 @@ struct walk_kernels
     if constexpr ( STORED ) return &k_batched< trav_item, stored_body< K, T >, kTravThreads, MB >;
     else return &k_batched< trav_item, traverse_body< K, T, VT >, kTravThreads, MB >;
   }
-  static cudaError_t setup()
-  {
-    if constexpr ( smem <= 47 * 1024 ) return cudaSuccess;
-    static std::atomic< unsigned long long > configured{ 0 };
-    int dev = 0;
-    cudaError_t e = cudaGetDevice( &dev );
-    if ( e != cudaSuccess ) return e;
-    const unsigned long long bit = 1ull << ( dev & 63 );
-    if ( configured.load() & bit ) return cudaSuccess;
-    e = cudaFuncSetAttribute( single(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
-    if ( e == cudaSuccess ) e = cudaFuncSetAttribute( batched(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem );
-    if ( e == cudaSuccess ) configured.fetch_or( bit );
-    return e;
-  }
   static cudaError_t launch(const trav_item &it, uint32_t grid, cudaStream_t s)
   {
-    const cudaError_t e = setup();
-    if ( e != cudaSuccess ) return e;
     single()<<< grid, kTravThreads, smem, s >>>( it );
     return cudaGetLastError();
   }
   static cudaError_t launch_batch(const batch_launch &b, cudaStream_t s)
   {
-    const cudaError_t e = setup();
-    if ( e != cudaSuccess ) return e;
     batched()<<< b.blocks, kTravThreads, smem, s >>>( static_cast< const trav_item * >( b.items ), b.starts, b.nitems );
     return cudaGetLastError();
   }
