@@ -72,8 +72,9 @@ struct object
   // test from the vertices instead of storing all of them.
   bool store_slabs = false;
   bool stored = false;  // the last build stored them
-  // The walk over stored slabs reached its stack bound on this object's tree: its traversals compute their slabs
-  // until the element count changes.
+  // False: a walk over stored slabs reached its stack bound on this object's tree, and its traversals compute their
+  // slabs until the element count changes. Defensive: the walk turns depth-first before its own bound, so only a bound
+  // lowered by the test hook (bvhg_test_dense_stack) is reached.
   bool dense_ok = true;
   // Patches (bvhg_cluster): valid until the next set_elements or rebuild.
   bool clustered = false;
@@ -616,7 +617,7 @@ bvhg_status find_pairs(bvhg_ctx *ctx, object &a, object &b, bool self, const uin
     if ( st != BVHG_OK ) return st;
     if ( ctx->host_ps->error == kErrOverflowStack && dense && a.stored && b.stored )
     {
-      // the walk over stored slabs reached its stack bound: search again with computed slabs
+      // the walk over stored slabs reached its (lowered) stack bound: search again with computed slabs
       a.dense_ok = false;
       b.dense_ok = false;
       continue;
@@ -1254,7 +1255,7 @@ bvhg_status run_batch(bvhg_ctx *ctx, const batch_args &x, uint64_t *counts)
       const pair_scalars &h = B.host_ps[sc];
       if ( h.error == kErrOverflowStack && ctx->objs[x.a[sc]]->dense_ok && ctx->objs[x.b[sc]]->dense_ok )
       {
-        // the walk over stored slabs reached its stack bound: this scene's objects compute their slabs and the
+        // the walk over stored slabs reached its (lowered) stack bound: this scene's objects compute their slabs and the
         // batch runs again (a new layout: the graph is captured again)
         ctx->objs[x.a[sc]]->dense_ok = false;
         ctx->objs[x.b[sc]]->dense_ok = false;
