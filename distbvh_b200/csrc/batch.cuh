@@ -48,7 +48,7 @@ __global__ void __launch_bounds__( THREADS, MIN_BLOCKS ) k_batched(const Args *_
 // waiting blocks take the place of the other object's kernels (1.3M and 1.0M triangles 526 -> 554 us with the chain, a
 // refit of 9.4M triangles 682 -> 713 us).
 constexpr uint64_t kChainElements = 1u << 19;
-constexpr uint32_t kChainBlocks = 296;  // a grid beyond it fills the device: its successor starts after it
+constexpr uint32_t kChainBlocks = 296;  // 2 blocks for each of 148 SMs: beyond it the successor's blocks start as these leave
 
 template< typename Args, void ( *Body )( const Args &, uint32_t, uint32_t ), int THREADS, int MIN_BLOCKS >
 __global__ void __launch_bounds__( THREADS, MIN_BLOCKS ) k_single(const Args a)

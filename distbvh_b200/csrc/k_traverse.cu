@@ -710,7 +710,10 @@ __device__ void stored_body(const trav_item &item, uint32_t bid, uint32_t)
 }
 
 // Shared memory per block of the walks, and their resident blocks per SM: as many as it allows (228 KB per SM, 1 KB of
-// it reserved per block) up to a cap that keeps the registers without spills.
+// it reserved per block) up to a cap on the registers. Most forms compile without spills at it; a few bytes are spilled
+// by the stored walks at 26-DOP and 18-DOP FP32 and by triangles at 26-DOP FP64 in sparse contact, and hexahedra in
+// sparse contact, whose slabs are formed from 24 coordinates in registers, spill 234 bytes at 26-DOP FP64 and 110 at
+// 18-DOP.
 template< int K, typename T, bool STORED >
 constexpr int kWalkSmem = ( kTravThreads / 32 ) * static_cast< int >( sizeof( walk_smem< K, T > ) );
 template< int K, typename T, bool STORED >
@@ -722,13 +725,15 @@ constexpr int kWalkBlocks = kWalkBySmem< K, T, STORED > < kWalkCap< K, T, STORED
                                                                                   : kWalkCap< K, T, STORED >;
 
 // One scene's item and grid. Dense contact: one warp per packet. Sparse: a persistent grid of at most the resident
-// blocks (4 per SM), one warp per chunk of 32 packets at most.
+// blocks (8 per SM), whose warps take chunks of 1 to 32 packets.
 //
 // Queries per packet in dense contact. A walk is a chain of steps: a small object whose packets of 32 do not fill the
-// device takes packets of one bucket (8), four times the warps with shorter chains. The line lies where those still run
-// at once (148 SMs x 16 warps): two plates of 1,600 / 10,000 triangles 64 / 91 -> 33 / 59 us, two blocks of 512 / 8,000
-// hexahedra 39 / 100 -> 22 / 54 us; beyond it the work of the narrow packets counts: 32,768 hexahedra 53 -> 64 us,
-// 70,000 tetrahedra against themselves 83 -> 113 us, and a batch, whose scenes share the device, 9.8 -> 13.3 ms.
+// device takes packets of one bucket (8), four times the warps with shorter chains. The line is where the narrow packets
+// fill the 16 warps per SM of the form with the fewest resident ones (26-DOP FP64; kWalkBlocks gives the others 20 to 32),
+// one line for all forms, found by measuring on both sides of it at 18- and 26-DOP FP64: two plates of 1,600 / 10,000
+// triangles 64 / 91 -> 33 / 59 us, two blocks of 512 / 8,000 hexahedra 39 / 100 -> 22 / 54 us; beyond it the work of the
+// narrow packets counts: 32,768 hexahedra 53 -> 64 us, 70,000 tetrahedra against themselves 83 -> 113 us, and a batch,
+// whose scenes share the device, 9.8 -> 13.3 ms.
 constexpr uint64_t kNarrowQueries = 148 * 16 * 8;
 
 template< int K, typename T >
