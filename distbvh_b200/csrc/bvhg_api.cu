@@ -1002,12 +1002,12 @@ bvhg_status capture_batch_fused(bvhg_ctx *ctx, batch_state &B, const batch_args 
     {
       uint2 *ex = B.exact.as< uint2 >() + B.off[sc];
       fg.recheck.push_back( recheck_args{ oa.verts, oa.V, ob.verts, ob.V, eps, cand, B.cap[sc], ex, B.cap[sc], ps + sc } );
-      fg.b_recheck.push_back( 1 );  // one launch divides all scenes' candidates
+      fg.b_recheck.push_back( scene_blocks( B.cap[sc] ) );
       fin = ex;
       cnt = &ps[sc].count2;
     }
     fg.gid.push_back( gid_args{ fin, cnt, B.cap[sc], oa.gid, ob.gid, self ? 1 : 0, B.out.as< uint64_t >() + 2 * B.off[sc] } );
-    fg.b_gid.push_back( 1 );
+    fg.b_gid.push_back( scene_blocks( B.cap[sc] ) );
   }
   // the tables on the device
   for ( auto &fg : grp )

@@ -414,8 +414,9 @@ struct recheck_args
   uint64_t cap;
   pair_scalars *ps;
 };
-// The scenes' rechecks, and below their id outputs, in one launch each over the resident blocks (items only: the
-// scenes' counts divide the work on the device).
+// The scenes' rechecks, and below their id outputs, in one launch each over at most the resident blocks (the scenes' counts
+// divide the work on the device). scene_blocks: the blocks that a scene's capacity can occupy.
+uint32_t scene_blocks(uint64_t cap);
 cudaError_t launch_recheck_batch(int K, uint32_t V, const batch_launch &b, cudaStream_t s);
 
 struct gid_args
