@@ -154,17 +154,17 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
 // element tests on all slabs for them, most on idle lanes.
 // What bounds it is the chain of dependent reads and the instructions per test, so a step reads all slabs of its nodes
 // or elements at once (one trip to memory per step) and compares without branches.
-// Traversal of the 256^3 lattice at 26-DOP FP64 25.6 -> 13.9 ms; 161^3 at 18-DOP FP32 2.53 -> 1.46 ms; 200,003
-// tetrahedra against themselves 208 -> 151 us; two plates of 10,000 triangles 186 -> 91 us; in sparse contact the
-// sphere on the plate (9.4M triangles) 105 -> 63 us. Measured and slower: the same expansion, then all 32 queries
-// against every bucket and four queries by eight elements per round from shared memory (15.4 ms); the same with a
-// second round for the non-cardinal slabs by (survivor, slab) lanes (29 ms); rows read five slabs at a time (20 to 50
-// ms, depending on the resident warps).
+// Traversal of the 256^3 lattice at 26-DOP FP64 25.6 -> 12.9 ms; 161^3 at 18-DOP FP32 2.53 -> 1.33 ms; 200,003
+// tetrahedra against themselves 208 -> 130 us; two plates of 10,000 triangles 186 -> 91 us (54 in narrow packets); in
+// sparse contact the sphere on the plate (9.4M triangles) 105 -> 59 us. Measured and slower: the same expansion, then all
+// 32 queries against every bucket and four queries by eight elements per round from shared memory (15.4 ms); the same
+// with a second round for the non-cardinal slabs by (survivor, slab) lanes (29 ms); rows read five slabs at a time (20 to
+// 50 ms, depending on the resident warps).
 // A packet whose ranks straddle a jump of the Morton curve, or whose elements lie far apart, or one of whose elements is
 // long, has a union box that says little: the check of the small children keeps its walk on the nodes that one of its
 // queries overlaps, and the buckets' queries keep the cardinal tests on those. (Testing all queries of the packet against
 // every gathered element: 300,000 triangles of which 100 span half the domain against 300,000 small ones 15.1 ms instead
-// of 8.6, one in 1,000 spanning 0.3 of it 2.8 instead of 1.6 ms, and the even tet lattices above 4-5% more of a step.)
+// of 8.6, one in 1,000 spanning 0.3 of it 2.8 instead of 1.6 ms, and the even lattices 13.9 and 1.46 ms.)
 //
 // The element slabs come from the rows that the slab kernel stored (STORED: dense contact; slab-major per bucket, so
 // that the filter reads the pairs of one slab of eight elements as one piece) or are computed from the vertices: the
