@@ -32,6 +32,10 @@ __device__ __forceinline__ void cp_async_wait_all()
   asm volatile( "cp.async.wait_all;" ::: "memory" );
 }
 
+// Closes a group of the copies issued since the last one; waits until at most the newest group is still in flight.
+__device__ __forceinline__ void cp_async_commit() { asm volatile( "cp.async.commit_group;" ::: "memory" ); }
+__device__ __forceinline__ void cp_async_wait_older() { asm volatile( "cp.async.wait_group 1;" ::: "memory" ); }
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
 {
   asm volatile( "mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"( smem_addr( bar ) ), "r"( count ) : "memory" );

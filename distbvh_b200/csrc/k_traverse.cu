@@ -139,8 +139,8 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
 //   - Expand: lane = (node, child). Up to 16 nodes are popped from the packet's stack; every lane tests one child's
 //     slabs against the packet's union box. A leaf bucket that passes goes onto the bucket list, an internal node back
 //     onto the stack; children smaller than half the packet's box go onto the check list first.
-//   - Check: lane = query. The cardinal slabs of the listed boxes are staged in shared memory, eight boxes at a time,
-//     and every lane tests its query against them. A child that no query overlaps is dropped, and a bucket is listed
+//   - Check: lane = query. The cardinal slabs of the listed boxes are staged in shared memory, eight boxes at a time
+//     with the next eight on their way, and every lane tests its query against them. A child that no query overlaps is dropped, and a bucket is listed
 //     with the queries that overlap it.
 //   - Filter: lane = element of four listed buckets. The elements that overlap the packet's union box are gathered, 16
 //     at a time, as rows in shared memory, and with them the queries of their buckets.
@@ -175,12 +175,12 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
 // entry per tree level (at most 95). kWalkStack entries therefore always suffice. A lower stack_limit (test hook) can
 // be reached: the walk raises kErrOverflowStack, and the host runs the pair search again with computed slabs.
 constexpr int kWalkDepth = 96;  // radix tree over 96-bit (key, rank) pairs: at most 95 internal levels
-constexpr int kWalkStack = 288;
+constexpr int kWalkStack = 284;
 constexpr int kCheckCap = 64;   // listed children: checked once more than 32 are held
 constexpr int kCheckRows = 8;   // boxes staged per check step
 constexpr int kLeafCap = 64;    // listed buckets: filtered once more than 32 are held
 constexpr int kGather = 16;     // elements gathered before they are tested
-constexpr int kSurvivors = 128;  // (query, element) pairs past the cardinal tests: tested once 32 are held
+constexpr int kSurvivors = 96;  // (query, element) pairs past the cardinal tests: tested once 32 are held
 constexpr int kPairBuf = 64;    // buffered pairs per warp: drained once more than 32 are held
 
 template< int K, typename T >
@@ -189,7 +189,7 @@ struct walk_smem
   // read as (min, max) pairs, and written by asynchronous copies of pairs
   alignas( 16 ) T q[32][K];             // slabs of the packet's queries
   alignas( 16 ) T e[kGather][K];        // slabs of the gathered elements
-  alignas( 16 ) T rows[kCheckRows][6];  // cardinal slabs of the boxes being checked
+  alignas( 16 ) T rows[2][kCheckRows][6];  // cardinal slabs of the boxes being checked and of the next ones
   alignas( 16 ) T g[K];                 // the packet's union box
   alignas( 16 ) uint2 out[kPairBuf];    // pairs found and not yet written
   int list[kCheckCap];                  // children to check: 2 * parent + side
@@ -569,22 +569,27 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
       nleaf += __popc( mb );
       continue;
     }
-    // check: lane = query, the listed boxes' cardinal slabs against every query of the packet
-    for ( int b0 = 0; b0 < nl && !full; b0 += kCheckRows )
+    // check: lane = query, the listed boxes' cardinal slabs against every query of the packet; the next boxes are on their
+    // way meanwhile
+    int link = 0, next_link = 0;  // of the child whose slab this lane copies
+    auto stage = [&](int b0, int buf) {
+      static_assert( kCheckRows * 3 <= 32, "one pair per lane" );
+      const int k = static_cast< int >( lane ) / 3, a = static_cast< int >( lane ) - 3 * k;
+      if ( k < min( kCheckRows, nl - b0 ) )
+      {
+        const int e = sm.list[b0 + k];
+        copy_pair( &sm.rows[buf][k][2 * a], x.nbox + static_cast< size_t >( e >> 1 ) * D * 4 + a * 4 + ( e & 1 ) * 2 );
+        next_link = __ldg( reinterpret_cast< const int * >( x.child ) + e );
+      }
+      cp_async_commit();
+    };
+    stage( 0, 0 );
+    for ( int b0 = 0, buf = 0; b0 < nl && !full; b0 += kCheckRows, buf ^= 1 )
     {
       const int nb = min( kCheckRows, nl - b0 );
-      int link = 0;  // of the child whose slab this lane copies
-      {
-        static_assert( kCheckRows * 3 <= 32, "one pair per lane" );
-        const int k = static_cast< int >( lane ) / 3, a = static_cast< int >( lane ) - 3 * k;
-        if ( k < nb )
-        {
-          const int e = sm.list[b0 + k];
-          copy_pair( &sm.rows[k][2 * a], x.nbox + static_cast< size_t >( e >> 1 ) * D * 4 + a * 4 + ( e & 1 ) * 2 );
-          link = __ldg( reinterpret_cast< const int * >( x.child ) + e );
-        }
-      }
-      cp_async_wait_all();
+      link = next_link;
+      stage( b0 + kCheckRows, buf ^ 1 );
+      cp_async_wait_older();
       __syncwarp();
       unsigned alive = in_root ? ( 1u << nb ) - 1u : 0u;
 #pragma unroll
@@ -596,7 +601,7 @@ __device__ __forceinline__ void walk_packet(const trav_args< T > &x, const uint3
         for ( int j = 0; j < kCheckRows; ++j )
         {
           T bl, bh;
-          shared_pair( &sm.rows[j][2 * a], bl, bh );
+          shared_pair( &sm.rows[buf][j][2 * a], bl, bh );
           const bool o = ( ql < bh ) & ( bl < qh );
           alive &= o ? ~0u : ~( 1u << j );
         }
