@@ -140,8 +140,8 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
 //     slabs against the packet's union box. A leaf bucket that passes goes onto the bucket list, an internal node back
 //     onto the stack; children smaller than half the packet's box go onto the check list first.
 //   - Check: lane = query. The cardinal slabs of the listed boxes are staged in shared memory, eight boxes at a time
-//     with the next eight on their way, and every lane tests its query against them. A child that no query overlaps is dropped, and a bucket is listed
-//     with the queries that overlap it.
+//     with the next eight on their way, and every lane tests its query against them. A child that no query overlaps is
+//     dropped, and a bucket is listed with the queries that overlap it.
 //   - Filter: lane = element of four listed buckets. The elements that overlap the packet's union box are gathered, 16
 //     at a time, as rows in shared memory, and with them the queries of their buckets.
 //   - Cardinal tests: lane = (query of two, gathered element), the element's cardinal slabs in registers, over those
@@ -154,8 +154,8 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
 // element tests on all slabs for them, most on idle lanes.
 // What bounds it is the chain of dependent reads and the instructions per test, so a step reads all slabs of its nodes
 // or elements at once (one trip to memory per step) and compares without branches.
-// Traversal of the 256^3 lattice at 26-DOP FP64 25.6 -> 12.9 ms; 161^3 at 18-DOP FP32 2.53 -> 1.33 ms; 200,003
-// tetrahedra against themselves 208 -> 130 us; two plates of 10,000 triangles 186 -> 91 us (54 in narrow packets); in
+// Traversal of the 256^3 lattice at 26-DOP FP64 25.6 -> 12.3 ms; 161^3 at 18-DOP FP32 2.53 -> 1.30 ms; 200,003
+// tetrahedra against themselves 208 -> 128 us; two plates of 10,000 triangles 186 -> 91 us (52 in narrow packets); in
 // sparse contact the sphere on the plate (9.4M triangles) 105 -> 59 us. Measured and slower: the same expansion, then all
 // 32 queries against every bucket and four queries by eight elements per round from shared memory (15.4 ms); the same
 // with a second round for the non-cardinal slabs by (survivor, slab) lanes (29 ms); rows read five slabs at a time (20 to
@@ -164,7 +164,9 @@ __device__ __forceinline__ trav_args< T > typed(const trav_item &it)
 // long, has a union box that says little: the check of the small children keeps its walk on the nodes that one of its
 // queries overlaps, and the buckets' queries keep the cardinal tests on those. (Testing all queries of the packet against
 // every gathered element: 300,000 triangles of which 100 span half the domain against 300,000 small ones 15.1 ms instead
-// of 8.6, one in 1,000 spanning 0.3 of it 2.8 instead of 1.6 ms, and the even lattices 13.9 and 1.46 ms.)
+// of 8.65, one in 1,000 spanning 0.3 of it 2.8 instead of 1.62 ms, and the even lattices 13.9 and 1.46 instead of 12.9
+// and 1.33 ms. Waiting for every eight boxes of a check: 8.65, 1.62, 12.9 and 1.33 ms instead of 8.47, 1.55, 12.3 and
+// 1.30.)
 //
 // The element slabs come from the rows that the slab kernel stored (STORED: dense contact; slab-major per bucket, so
 // that the filter reads the pairs of one slab of eight elements as one piece) or are computed from the vertices: the
@@ -734,8 +736,8 @@ constexpr int kWalkBlocks = kWalkBySmem< K, T, STORED > < kWalkCap< K, T, STORED
 //
 // Queries per packet in dense contact. A walk is a chain of steps: a small object whose packets of 32 do not fill the
 // device takes packets of one bucket (8), four times the warps with shorter chains. The line is where the narrow packets
-// fill the 16 warps per SM of the form with the fewest resident ones (26-DOP FP64; kWalkBlocks gives the others 20 to 32),
-// one line for all forms, found by measuring on both sides of it at 18- and 26-DOP FP64: two plates of 1,600 / 10,000
+// fill the 16 warps per SM of the form with the fewest resident ones (26-DOP FP64; kWalkBlocks gives the others 20 to
+// 32), one line for all forms, found by measuring on both sides of it at 18- and 26-DOP FP64: two plates of 1,600 / 10,000
 // triangles 64 / 91 -> 33 / 59 us, two blocks of 512 / 8,000 hexahedra 39 / 100 -> 22 / 54 us; beyond it the work of the
 // narrow packets counts: 32,768 hexahedra 53 -> 64 us, 70,000 tetrahedra against themselves 83 -> 113 us, and a batch,
 // whose scenes share the device, 9.8 -> 13.3 ms.
